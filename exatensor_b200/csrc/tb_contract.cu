@@ -1,6 +1,6 @@
 // tb_contract.cu -- tensor contraction driver: D = beta*D + alpha*op(L)*op(R).
 //
-// Two executions of the same contraction:
+// Three executions of the same contraction:
 //  * TB_METHOD_TTGT ("plain", the reference's scheme in
 //    TALSH/tensor_algebra_gpu_nvidia.cu:5847-7188): permute L and R into
 //    K-major matrices, GEMM in the tensor's own data type, then permute the
@@ -9,10 +9,13 @@
 //  * TB_METHOD_FUSED (tb_tc.cu): the operand gathers fuse the input
 //    permutations with the conversion to tensor-core formats and the epilogue
 //    writes D through the output permutation with alpha/beta applied.
+//  * the one-kernel form (tb_direct.cu): the plain method's arithmetic without
+//    its permutation passes, for what TB_METHOD_AUTO would run as TTGT.
 // A full contraction into a scalar (D rank 0) uses a deterministic two-pass
 // dot-product kernel (the reference's gpu_array_dot_product__, :531).
 #include "tb_common.cuh"
 #include "tb_contract.h"
+#include "tb_direct.h"
 #include "tb_gemm.h"
 #include "tb_pattern.h"
 #include "tb_permute.cuh"
@@ -347,6 +350,29 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
     unsigned tune = 0;
     uint64_t key = 0;
     descriptor_of(Z, dtk, f);
+    // The plain method in one kernel, in the tensors' own layouts: the same FP64
+    // or wider sums without the permutation passes and their scratch.  On random
+    // contractions of the four kinds it ran 1.1 to 7 times as fast as TTGT (8 to
+    // 30 us instead of 27 to 100 us for small ones).  TTGT keeps the products
+    // that the FP64 tensor rate bounds, where its larger tiles read the operands
+    // less often (1980 x 1881 x 816: 327 us against 342 us).  Where the tensor
+    // cores are picked, one kernel still replaces them when it is predicted to
+    // take less than their launches alone: about 16 kernels, 60 us or more for
+    // the smallest product (K = 9856, M = N = 150: 147 us against 67 us), unless
+    // the plan asks for details of that path.
+    auto try_direct = [&](int picked, int* err) {
+      constexpr double kFusedLaunchesUs = 50.0;
+      const bool asked = plan && (plan->slices || plan->tile_n || plan->tile_m || plan->bf16_terms || plan->moduli);
+      if (picked == TB_METHOD_FUSED && asked) return false;
+      if (picked == TB_METHOD_TTGT && dtk == kR8 && Z.M >= 1792 && Z.N >= 1792 && Z.K >= 512) return false;
+      DirectPlan dp;
+      if (direct_plan(Z, dtk, d, l, r, &dp) != 0) return false;
+      if (picked == TB_METHOD_FUSED && dp.us >= kFusedLaunchesUs) return false;
+      g_stats.method = TB_METHOD_TTGT;
+      g_stats.gemm_launches = 1;
+      *err = run_direct(dp, dtk, cplx ? ar : real_alpha(ar, ai), cplx ? ai : 0.0, accumulative != 0, lconj, rconj, s);
+      return true;
+    };
     auto candidate = [&](int c) {
       tb_plan_t cp = plan ? *plan : tb_plan_t{};
       cp.method = c == 0 ? TB_METHOD_TTGT : TB_METHOD_FUSED;
@@ -414,11 +440,14 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
         g_stats.m = Z.M; g_stats.n = Z.N; g_stats.k = Z.K;
         g_stats.flops = (cplx ? 8.0 : 2.0) * (double)Z.M * (double)Z.N * (double)Z.K;
       }
+      const bool mine = !selector_is_callers();
+      if ((idx == 0 || mine) && try_direct(idx == 0 ? TB_METHOD_TTGT : TB_METHOD_FUSED, &e)) return e;
       learned = candidate(idx);
       return run_method(Z, dtk, ddims, d, ldims, l, rdims, r, ar, ai, accumulative, lconj, rconj, &learned, s,
                         /*fallback=*/true);
     }
     method = select_method(dtk, Z, plan);
+    if (try_direct(method, &e)) return e;
   }
   if (method == TB_METHOD_AUTO) method = TB_METHOD_TTGT;
   learned = plan ? *plan : tb_plan_t{};

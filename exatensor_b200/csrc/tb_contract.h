@@ -36,6 +36,9 @@ constexpr int kNumCandidates = 5;
 // tune_mask: candidates to time before choosing (0: none).
 int selector_pick(const float* features, int* idx, unsigned* tune_mask, uint64_t* key);
 void selector_remember(uint64_t key, int idx);
+// Whether the caller installed the network in use: its choice of the tensor
+// cores then stands, where the library would refine its own network's.
+bool selector_is_callers();
 void selector_autoload();
 
 }  // namespace tb

@@ -1,0 +1,16 @@
+// tb_direct.h -- one-kernel contractions in the tensors' own layouts (tb_direct.cu).
+#pragma once
+#include <cuda_runtime.h>
+
+#include "tb_direct_plan.h"
+
+namespace tb {
+
+// plan_direct over the kernels' tile shapes on the current device.
+int direct_plan(const Matricization& Z, int dtk, const void* d, const void* l, const void* r, DirectPlan* out,
+                int force_variant = -1, int force_split = 0, int force_box = -1);
+// Launches it; alpha as the plain method takes it (real kinds: ai = 0).
+int run_direct(const DirectPlan& plan, int dtk, double ar, double ai, bool accumulate, int lconj, int rconj,
+               cudaStream_t s);
+
+}  // namespace tb

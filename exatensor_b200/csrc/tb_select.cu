@@ -50,6 +50,7 @@ bool in_matrix_order(const std::vector<MGroup>& first, const std::vector<MGroup>
 struct Selector {
   std::mutex mu;
   bool on = false;
+  bool shipped = false;  // the weights that came with the library (else the caller's own)
   int nh = 0;
   std::vector<float> p, mean, scale;
   float margin = 0.f;
@@ -185,6 +186,12 @@ int selector_pick(const float* f, int* idx, unsigned* tune_mask, uint64_t* key) 
   return 0;
 }
 
+bool selector_is_callers() {
+  Selector& S = sel();
+  std::lock_guard<std::mutex> lk(S.mu);
+  return S.on && !S.shipped;
+}
+
 void selector_remember(uint64_t key, int idx) {
   Selector& S = sel();
   std::lock_guard<std::mutex> lk(S.mu);
@@ -213,6 +220,7 @@ extern "C" int tb_selector_install(int n_hidden, const float* params, const floa
   std::lock_guard<std::mutex> lk(S.mu);
   S.cache.clear();
   S.seen.clear();
+  S.shipped = false;
   if (!params) { S.on = false; return 0; }
   if (n_hidden < 1 || n_hidden > 4096 || !mean || !scale) {
     set_error("tb_selector_install: bad arguments (hidden units 1..4096)");
@@ -312,7 +320,13 @@ void selector_autoload() {
     FILE* f = std::fopen(path.c_str(), "rb");
     if (!f) return;
     std::fclose(f);
-    if (tb_selector_load(path.c_str())) set_error("");  // a bad file leaves the size rule in place
+    if (tb_selector_load(path.c_str())) {
+      set_error("");  // a bad file leaves the size rule in place
+    } else if (!(env && *env)) {
+      Selector& S = sel();
+      std::lock_guard<std::mutex> lk(S.mu);
+      S.shipped = S.on;
+    }
   });
 }
 }  // namespace tb

@@ -1,0 +1,75 @@
+"""CPU replay of the one-kernel contraction's plan and index arithmetic
+(tests/emul/direct_emul.cpp): random patterns, extents with remainders, every
+tile shape, K split and row box, in exact integers against plain loops."""
+import os
+import random
+import subprocess
+
+import pytest
+
+import oracle as O
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(HERE, "..", "exatensor_b200", "csrc")
+PATTERNS = ["D(a,b,i,j)+=L(a,b,c,d)*R(c,d,i,j)", "D(a,i,b,j)+=L(a,k,c,i)*R(c,b,k,j)",
+            "D(a,b,c,d)+=L(c,k,a,l)*R(l,d,k,b)", "D(a,b,c,d,e,f)+=L(d,e,g,a)*R(g,f,b,c)",
+            "D(a,b,c,d)+=L(d,b,e,a)*R(e,c)", "D(a,b,c)+=L(d,c,a)*R(b,d)", "D(a,b,c,d)+=L(e,b)*R(a,e,c,d)",
+            "D(a,b)+=L(a,c,d)*R(d,b,c)", "D(a)+=L(k,a)*R(k)", "D(a,b)+=L(b)*R(a)", "D(a,b)+=L()*R(b,a)"]
+
+
+@pytest.fixture(scope="module")
+def emul(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("direct") / "direct_emul")
+    subprocess.run(["g++", "-O2", "-std=c++17", os.path.join(HERE, "emul", "direct_emul.cpp"),
+                    os.path.join(CSRC, "tb_direct_plan.cpp"), os.path.join(CSRC, "tb_pattern.cpp"), "-o", exe],
+                   check=True)
+    return exe
+
+
+def labels(pattern):
+    return [[x for x in part.split(")")[0].split(",") if x] for part in pattern.split("(")[1:]]
+
+
+def test_shapes_match_the_kernels():
+    """The shapes in the emulation are those the launch table instantiates."""
+    src = open(os.path.join(CSRC, "tb_direct.cu")).read()
+    import re
+    v = [tuple(int(x) for x in m) for m in re.findall(r"Variant<E, (\d+), (\d+), (\d+), (\d+), (\d+), (\d+), \d+, (\d+)>", src)]
+    got = [(wm * mi * 8, wn * ni * 8, bk * kw, wm * wn * kw * 32, occ) for wm, wn, kw, mi, ni, bk, occ in v]
+    em = open(os.path.join(HERE, "emul", "direct_emul.cpp")).read()
+    want = [tuple(int(x) for x in m) for m in re.findall(r"\{(\d+), (\d+), (\d+), (\d+), (\d+)\}", em)]
+    assert got == want
+
+
+def test_every_index_once(emul):
+    rng = random.Random(5)
+    lines = []
+    for n in range(420):
+        pat = rng.choice(PATTERNS)
+        d, l, r = labels(pat)
+        ext = {x: rng.choice([1, 2, 3, 5, 7, 8, 11, 16, 17, 19, 23, 33]) for x in set(d + l + r)}
+        dims = [[ext[x] for x in g] for g in (d, l, r)]
+        while True:  # bounded work for the plain loops
+            work = 1
+            for x in ext.values():
+                work *= x
+            if work <= 600000:
+                break
+            big = max(ext, key=ext.get)
+            ext[big] = max(1, ext[big] // 2)
+            dims = [[ext[x] for x in g] for g in (d, l, r)]
+        cp = O.parse_pattern(pat)[0]
+        cplx = rng.random() < 0.3
+        es = rng.choice([8, 16] if cplx else [4, 8])
+        force = rng.random() < 0.75
+        variant = rng.randrange(6 if cplx else 7) if force else -1
+        split = rng.choice([1, 2, 4, 8]) if force and rng.random() < 0.5 else 0
+        box = rng.choice([0, 1]) if force else -1
+        flat = [len(d), len(l), len(r)] + [x for g in dims for x in g] + list(cp) + [es, int(cplx), variant, split, box]
+        lines.append(" ".join(map(str, flat)))
+    out = subprocess.run([emul], input="\n".join(lines), capture_output=True, text=True, check=True).stdout.splitlines()
+    assert len(out) == len(lines)
+    bad = [(i, o) for i, o in zip(lines, out) if o.startswith("BAD")]
+    assert not bad, bad[:5]
+    ok = [o for o in out if o.startswith("OK")]
+    assert len(ok) > 150 and any("box=1" in o for o in ok) and any("split=8" in o for o in ok)
