@@ -148,9 +148,10 @@ u128 moduli_product(int n) {
   return M;
 }
 
-// The largest p with M > 2 Kr 2^(2p) for n moduli (checked in exact integer arithmetic).
+// The largest p with M (1 - 2^-20) > 2 Kr 2^(2p) for n moduli (checked in exact
+// integer arithmetic; the 2^-20 is the room that crt_kernel's quotient needs).
 int residue_bits(int n, int64_t Kr) {
-  const u128 M = moduli_product(n);
+  const u128 Mf = moduli_product(n), M = Mf - (Mf >> 20);
   int p = 0;
   while (p < 60 && (M >> (2 * (p + 1))) > (u128)(2 * Kr)) ++p;
   return p;
@@ -184,12 +185,16 @@ bool plan_residues(int64_t Kr, int want, ResiduePlan* out) {
   R.rs.pscale = std::ldexp(1.0, p + 1);
   const u128 M = moduli_product(n);
   R.crt.n = n;
-  R.crt.M_lo = (uint64_t)M;
-  R.crt.M_hi = (uint64_t)(M >> 64);
-  R.crt.Md = (double)(uint64_t)(M >> 64) * 18446744073709551616.0 + (double)(uint64_t)M;
   R.crt.shift = 2 * (p + 1);
   R.rs.p = p;
   R.rs.ndig = p <= 46 ? 3 : 4;
+  int b = 0;
+  while (b < 127 && (M >> b) != 0) ++b;
+  // bits [b - 41 (k + 1), b - 41 k) of x, k = 0..2, as a double (exact)
+  auto part = [&](u128 x, int k) {
+    const int lo = std::max(0, b - 41 * (k + 1)), hi = std::max(0, b - 41 * k);
+    return std::ldexp((double)(uint64_t)((x >> lo) & (((u128)1 << (hi - lo)) - 1)), lo);
+  };
   for (int i = 0; i < n; ++i) {
     const int m = kModuliTable[i];
     const u128 Mi = M / (u128)m;
@@ -198,10 +203,15 @@ bool plan_residues(int64_t Kr, int want, ResiduePlan* out) {
     for (int c = 1; c < m; ++c)
       if ((mi_mod * c) % m == 1) { y = c; break; }
     R.crt.mod[i] = m;
-    R.crt.y[i] = y;
-    R.crt.mi_lo[i] = (uint64_t)Mi;
-    R.crt.mi_hi[i] = (uint64_t)(Mi >> 64);
+    const u128 s = Mi * (u128)y;
+    R.crt.s1[i] = part(s, 0);
+    R.crt.s2[i] = part(s, 1);
+    R.crt.s3[i] = part(s, 2);
   }
+  R.crt.M1 = part(M, 0);
+  R.crt.M2 = part(M, 1);
+  R.crt.M3 = part(M, 2);
+  R.crt.invM = 1.0 / (double)M;
   return true;
 }
 
@@ -470,7 +480,7 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
     P.nf_skip = resid ? 0 : 1;  // residues: crt_kernel leaves the flagged entries to the fix-up
     if (resid) {
       P.res = (uint8_t*)(ws + offRES);
-      P.res_ld = Mpad;
+      P.res_ld = Npad;
       P.res_plane = Npad * Mpad;
     }
     // Work units: dynamic (a counter) unless TB_TC_SCHED=0.  L2 policy: with
@@ -492,21 +502,18 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
       // Chinese remainder reconstruction of the exact products into D
       CrtParams C = RP.crt;
       C.res = (const uint8_t*)(ws + offRES);
-      C.res_ld = Mpad;
+      C.res_ld = Npad;
       C.res_plane = Npad * Mpad;
       C.rows = M;
       C.cols = Nc;
       C.dm = dm; C.dn = dn; C.D = d;
       C.rowexp = rowx; C.colexp = colx;
       C.ar = realpha; C.ai = cplx ? ai : 0.0; C.br = P.br; C.bi = 0.0;
-      static DeviceOnce crt_attr_r, crt_attr_c;
-      const cudaError_t ea = cplx ? smem_limit_once(crt_attr_c, crt_kernel<true>, kCrtTableBytes)
-                                  : smem_limit_once(crt_attr_r, crt_kernel<false>, kCrtTableBytes);
-      if (ea != cudaSuccess) { set_error("residue reconstruction smem attribute: %s", cudaGetErrorString(ea)); err = TB_ERR_CUDA; break; }
-      const int64_t groups = Nc;  // column groups of crt_kernel (one D column each)
-      const unsigned cg = (unsigned)std::max<int64_t>(1, std::min<int64_t>(groups, 3 * num_sms()));
-      if (cplx) crt_kernel<true><<<cg, 256, kCrtTableBytes, s>>>(C);
-      else crt_kernel<false><<<cg, 256, kCrtTableBytes, s>>>(C);
+      const int64_t rb = (M + 31) / 32, cb = (Nr + kCrtCols * kCrtWarps - 1) / (kCrtCols * kCrtWarps);
+      if (rb * cb > INT32_MAX) { set_error("residue reconstruction grid too large"); err = TB_ERR_LIMIT; break; }
+      const unsigned cg = (unsigned)(rb * cb);
+      if (cplx) crt_kernel<true><<<cg, 32 * kCrtWarps, 0, s>>>(C);
+      else crt_kernel<false><<<cg, 32 * kCrtWarps, 0, s>>>(C);
       count_launch();
       if (cudaError_t e = cudaGetLastError()) {
         set_error("residue reconstruction launch: %s", cudaGetErrorString(e));

@@ -32,8 +32,9 @@ constexpr int kTcThreads = 192;
 
 // EPI_RESID: modular residues (Ozaki scheme II) -- each pass is one modulus
 // (pass_shift holds it) and the epilogue stores acc mod m as one byte per
-// element into residue plane `pass` (layout [pass][column][row], rows fastest);
-// crt_kernel later rebuilds D from all planes.
+// element into residue plane `pass` (layout [pass][row][column], columns
+// fastest: a thread holds one row of the accumulator, so 32 columns are two
+// 16-byte stores); crt_kernel later rebuilds D from all planes.
 enum TcEpilogue { EPI_OZAKI_R = 0, EPI_OZAKI_C = 1, EPI_BF16_R = 2, EPI_BF16_C = 3, EPI_RESID = 4 };
 
 struct __align__(64) TcGemmParams {
@@ -57,7 +58,7 @@ struct __align__(64) TcGemmParams {
   unsigned int* err;
   int nf_skip;                // 1: leave entries of flagged rows / columns to the non-finite fix-up
   uint8_t* res;               // EPI_RESID: residue planes
-  int64_t res_ld, res_plane;  // EPI_RESID: column stride and plane stride (bytes)
+  int64_t res_ld, res_plane;  // EPI_RESID: row stride and plane stride (bytes)
   int res_nch;                // EPI_RESID: passes per modulus (K chunks of at most
                               // 1023 blocks each, added up mod m by the epilogue)
   unsigned int* sched;        // single-SM kernel: zeroed work-unit counter (dynamic
@@ -155,30 +156,47 @@ __device__ __forceinline__ void epilogue_pass(const EP& P, uint32_t tcol, bool m
     tmem_ld32(tcol + (uint32_t)(c * 32), r);
     const int n0 = nb * BN + c * 32;
     if constexpr (EPI == EPI_RESID) {
-      // residues of the exact INT32 sums: shift is the modulus m, and the
-      // caller passes this pass's plane through P.res / res_plane.  v mod m
-      // by a multiply-high with magic = floor(2^32 / m): the quotient estimate
-      // is off by at most one either way, so two conditional corrections give
-      // the residue in [0, m) (integer pipes only; no division).  Later K
-      // chunks of a modulus (!first) add their residue to the stored one.
+      // residues of the exact INT32 sums: shift is the modulus m, and dmo the
+      // offset of this thread's row in the modulus's plane.  v + bias, bias the
+      // smallest multiple of m from 2^31 on, is v's class as an unsigned number
+      // (|v| <= 2^31 - 2^21, so it does not wrap); its quotient by a
+      // multiply-high with magic = floor(2^32 / m) is exact or one short, which
+      // one unsigned minimum corrects (no division, no branches).  Padded rows
+      // and columns of the plane are written too.  Later K chunks of a modulus
+      // (!first) add their residue to the stored one.  With one byte store per
+      // element this epilogue bounded K = 1600 products (102 us for 1600^2 x 15
+      // moduli); packed it hides behind the next unit's MMAs.
       if constexpr (std::is_same<EP, TcGemmParams>::value) {
-        if (mval) {
-          uint8_t* col = P.res + dmo;  // dmo: this modulus's plane offset + row
+        const uint32_t m = (uint32_t)shift, bias = ((0x80000000u + m - 1) / m) * m;
+        auto residue = [&](uint32_t v) {
+          v += bias;
+          const uint32_t x = v - __umulhi(v, (uint32_t)magic) * m;
+          return min(x, x - m);
+        };
+        uint4* dst = reinterpret_cast<uint4*>(P.res + dmo + n0);
+        uint32_t w[8];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (n0 + j >= P.N) break;
-            const int v = (int)r[j];
-            int rr = v - __mulhi(v, magic) * shift;
-            rr += rr < 0 ? shift : 0;
-            rr -= rr >= shift ? shift : 0;
-            uint8_t* dst = col + (int64_t)(n0 + j) * P.res_ld;
-            if (!first) {
-              rr += *dst;
-              rr -= rr >= shift ? shift : 0;
+        for (int q = 0; q < 8; ++q) {
+          const uint32_t lo = __byte_perm(residue(r[4 * q]), residue(r[4 * q + 1]), 0x0040);
+          const uint32_t hi = __byte_perm(residue(r[4 * q + 2]), residue(r[4 * q + 3]), 0x0040);
+          w[q] = __byte_perm(lo, hi, 0x5410);
+        }
+        if (!first) {
+          const uint4 o0 = dst[0], o1 = dst[1];
+          const uint32_t o[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            uint32_t s = 0;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              const uint32_t x = ((w[q] >> (8 * t)) & 255u) + ((o[q] >> (8 * t)) & 255u);
+              s |= min(x, x - m) << (8 * t);
             }
-            *dst = (uint8_t)rr;
+            w[q] = s;
           }
         }
+        dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
       }
       continue;
     }
@@ -397,9 +415,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
         tc_fence_after();
         const bool first = EPI == EPI_RESID ? (p - w.p0 == 0) : (p == 0);
         const int shift = (EPI == EPI_OZAKI_R || EPI == EPI_OZAKI_C || EPI == EPI_RESID) ? P.pass_shift[p] : 0;
-        const int64_t dmp = EPI == EPI_RESID ? (int64_t)(p / P.res_nch) * P.res_plane + m : dmo;
+        const int64_t dmp = EPI == EPI_RESID ? (int64_t)(p / P.res_nch) * P.res_plane + (int64_t)m * P.res_ld : dmo;
         epilogue_pass<BN, EPI>(P, tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN),
-                               EPI == EPI_RESID ? m < P.M : mval, dmp, re, nb, first, shift,
+                               mval, dmp, re, nb, first, shift,
                                EPI == EPI_RESID ? P.pass_magic[p] : 0);
         tc_fence_before();
         __syncwarp();
@@ -552,9 +570,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
         if (!(ok = mbar_wait_warp(&bars->acc_full[a], aph, P.err, 1u, kEpilogueSleepNs))) break;
         tc_fence_after();
         const int shift = (EPI == EPI_OZAKI_R || EPI == EPI_OZAKI_C || EPI == EPI_RESID) ? P.pass_shift[p] : 0;
-        const int64_t dmp = EPI == EPI_RESID ? (int64_t)(p / P.res_nch) * P.res_plane + m : dmo;
+        const int64_t dmp = EPI == EPI_RESID ? (int64_t)(p / P.res_nch) * P.res_plane + (int64_t)m * P.res_ld : dmo;
         epilogue_pass<BN, EPI>(P, tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN),
-                               EPI == EPI_RESID ? m < P.M : mval, dmp, re, nb,
+                               mval, dmp, re, nb,
                                EPI == EPI_RESID ? (p - w.p0 == 0) : (p == 0), shift,
                                EPI == EPI_RESID ? P.pass_magic[p] : 0);
         tc_fence_before();

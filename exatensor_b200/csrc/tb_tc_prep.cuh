@@ -691,22 +691,27 @@ __global__ void __launch_bounds__(256) nonfinite_fixup_kernel(const __grid_const
 
 
 // ---- Ozaki scheme II reconstruction (Chinese remainder theorem) ------------------
-// With M = prod m_i, M_i = M / m_i and y_i = M_i^-1 mod m_i, the exact integer
-// dot product is C = sum_i t_i M_i mod M, t_i = (r_i y_i) mod m_i, taken in the
-// symmetric range (|C| < M / 2 by the choice of p).  Each t_i M_i < M, so the
-// sum stays below n M < 2^123 in 128 bits.  C is converted to FP64 (about one
-// rounding), scaled by 2^(e_m + f_n - 2(p+1)) exactly, and D = beta D +
-// alpha C through the offset tables.  Rows and columns flagged as holding a
-// NaN or an infinity are left to the fix-up kernel.  Persistent CTAs take
-// whole columns, threads along the rows (D's fastest).
+// With M = prod m_i, M_i = M / m_i, y_i = M_i^-1 mod m_i and s_i = y_i M_i, the
+// exact integer dot product is C = sum_i r_i s_i - Q M, |C| < M / 2 by the choice
+// of p.  s_i and M are cut into three parts of at most 41 bits of 2^b > M, so
+// that each part's sum over r_i < 2^8 and 15 terms, and its difference with Q
+// times M's part, is exact in FP64; the three differences are added with one
+// error term, so C comes out within about one rounding whatever cancels.  Q =
+// rint(first sum / M) is right because |C| stays a part in 2^20 below M / 2
+// (residue_bits) and the dropped parts are below 2^-28 M.  C is scaled by 2^(e_m
+// + f_n - 2(p+1)) exactly, and D = beta D + alpha C through the offset tables.
+// Rows and columns flagged as holding a NaN or an infinity are left to the
+// fix-up kernel.  Bound by the bytes of the planes and D and by the FP64 units
+// (four operations per residue) about alike.  A 60 KB shared-memory table of
+// 128-bit multiples, one random 16-byte read per residue, took 80 us for 1600^2
+// x 15 moduli and 2.6 ms for 36864 x 2304 x 14.
 struct CrtParams {
-  const uint8_t* res;          // residue planes [i][column][row], bytes
+  const uint8_t* res;          // residue planes [i][row][column], bytes
   int64_t res_ld, res_plane;
   int n;
-  int mod[kMaxModuli], y[kMaxModuli];
-  uint64_t mi_lo[kMaxModuli], mi_hi[kMaxModuli];
-  uint64_t M_lo, M_hi;
-  double Md;                   // M as a double
+  int mod[kMaxModuli];
+  double s1[kMaxModuli], s2[kMaxModuli], s3[kMaxModuli];
+  double M1, M2, M3, invM;
   int64_t rows, cols;          // rows of A; columns of B (complex: column pairs)
   const int64_t* dm;
   const int64_t* dn;
@@ -717,114 +722,88 @@ struct CrtParams {
   double ar, ai, br, bi;
 };
 
-__device__ __forceinline__ double u128_to_double(unsigned __int128 x) {
-  return (double)(uint64_t)(x >> 64) * 18446744073709551616.0 + (double)(uint64_t)x;
-}
+// A warp takes 32 rows (lanes; D's fastest) and a thread kCrtCols residue
+// columns of its row, one 16-byte load per plane; the warps of a CTA take
+// neighbouring columns, so that together they use whole lines of the planes.
+constexpr int kCrtCols = 16, kCrtWarps = 4;
 
-// The table of crt_kernel: entry i * 256 + r = ((r y_i) mod m_i) M_i (r < m_i),
-// built by each CTA in shared memory, so that a residue costs one lookup and a
-// 128-bit addition.
-constexpr int kCrtTableBytes = kMaxModuli * 256 * 16;
-struct alignas(16) CrtEntry { uint64_t lo, hi; };
-
-// Residues of the four D entries (col, m .. m + 3) from the n planes: one
-// 32-bit load per plane (m a multiple of 4; the planes' row length and plane
-// stride are multiples of 4 bytes, so the words are aligned and lie inside the
-// padded plane even past the last row), byte t of word i holding residue i of
-// row m + t.
-__device__ __forceinline__ void crt_load4(const CrtParams& P, int64_t col, int64_t m, uint32_t (&w)[kMaxModuli]) {
-  const uint8_t* rp = P.res + col * P.res_ld + m;
-#pragma unroll
-  for (int i = 0; i < kMaxModuli; ++i) w[i] = i < P.n ? *reinterpret_cast<const uint32_t*>(rp + i * P.res_plane) : 0u;
-}
-__device__ __forceinline__ void crt_byte(const uint32_t (&w)[kMaxModuli], int t, uint32_t (&r)[kMaxModuli]) {
-#pragma unroll
-  for (int i = 0; i < kMaxModuli; ++i) r[i] = __byte_perm(w[i], 0u, 0x4440 + t);
-}
-
-// The exact integer from its residues, in FP64 (about one rounding).
-__device__ __forceinline__ double crt_combine(const CrtParams& P, const CrtEntry* tab, const uint32_t (&r)[kMaxModuli]) {
-  uint64_t lo = 0, hi = 0;
-#pragma unroll
-  for (int i = 0; i < kMaxModuli; ++i) {
-    if (i >= P.n) break;
-    const CrtEntry t = tab[i * 256 + r[i]];
-    lo += t.lo;
-    hi += t.hi + (lo < t.lo ? 1u : 0u);
-  }
-  unsigned __int128 S = ((unsigned __int128)hi << 64) | lo;
-  const unsigned __int128 M = ((unsigned __int128)P.M_hi << 64) | P.M_lo;
-  // S < n M: subtract q M, q = floor(S / M) estimated in FP64 (within one), then
-  // at most a few exact corrections
-  uint64_t q = (uint64_t)(u128_to_double(S) / P.Md);
-  if (q > 0) --q;
-  S -= (unsigned __int128)q * M;
-  for (int it = 0; it < 4 && S >= M; ++it) S -= M;
-  const bool neg = S > (M >> 1);
-  const double v = u128_to_double(neg ? M - S : S);
-  return neg ? -v : v;
-}
-
-// Each CTA takes residue columns (one real D column, or one complex one: its
-// two residue columns) and each thread, for every four consecutive rows it
-// owns, loads one word per plane -- the residues of all four rows -- before
-// combining them.  (One byte load per plane and row kept four times as many
-// loads in flight for the same bytes; four columns per group took 113
-// registers and ran 8% slower.)
 template <bool CPLX>
-__global__ void __launch_bounds__(256) crt_kernel(const __grid_constant__ CrtParams P) {
-  extern __shared__ __align__(16) unsigned char crt_smem[];
-  CrtEntry* tab = reinterpret_cast<CrtEntry*>(crt_smem);
-  for (int e = threadIdx.x; e < P.n * 256; e += blockDim.x) {
-    const int i = e >> 8, r = e & 255;
-    CrtEntry t{0, 0};
-    if (r < P.mod[i]) {
-      const uint64_t c = (uint64_t)((r * P.y[i]) % P.mod[i]);
-      const unsigned __int128 v = (unsigned __int128)c * (((unsigned __int128)P.mi_hi[i] << 64) | P.mi_lo[i]);
-      t.lo = (uint64_t)v;
-      t.hi = (uint64_t)(v >> 64);
+__global__ void __launch_bounds__(32 * kCrtWarps, 3) crt_kernel(const __grid_constant__ CrtParams P) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned row_blocks = (unsigned)((P.rows + 31) / 32);
+  const unsigned cb = blockIdx.x / row_blocks, rb = blockIdx.x - cb * row_blocks;
+  const int64_t m = (int64_t)rb * 32 + lane;
+  constexpr int RC = CPLX ? 2 : 1, DC = kCrtCols / RC;  // residue columns per D column; D columns per thread
+  const int64_t rcols = P.cols * RC;
+  const int64_t c0 = ((int64_t)cb * kCrtWarps + warp) * kCrtCols;
+  if (c0 >= rcols || m >= P.rows) return;
+  const int re = P.rowexp[m];
+  if (re >= kNonFiniteExp) return;  // flagged row: the fix-up's
+  const uint8_t* rp = P.res + m * P.res_ld + c0;  // rows are padded to whole column tiles: always inside the plane
+  uint4 w[kMaxModuli];
+#pragma unroll
+  for (int i = 0; i < kMaxModuli; ++i)
+    w[i] = i < P.n ? *reinterpret_cast<const uint4*>(rp + i * P.res_plane) : make_uint4(0, 0, 0, 0);
+  const int64_t dmo = P.dm[m];
+  const bool read_d = P.br != 0.0 || P.bi != 0.0;
+  using E = typename std::conditional<CPLX, double2, double>::type;
+  E* D = (E*)P.D;
+  constexpr int G = 8, H = G / RC;  // residue columns and D columns of one group
+#pragma unroll
+  for (int g = 0; g < kCrtCols / G; ++g) {
+    E old[H];
+    int64_t o[H];
+    int ce[H];
+#pragma unroll
+    for (int j = 0; j < H; ++j) {
+      const int64_t n = c0 / RC + g * H + j;
+      o[j] = -1;
+      if (n >= P.cols) continue;
+      ce[j] = P.colexp[n * RC];
+      if (ce[j] >= kNonFiniteExp) continue;  // flagged column: the fix-up's
+      o[j] = dmo + P.dn[n];
+      if (read_d) old[j] = D[o[j]];
     }
-    tab[e] = t;
-  }
-  __syncthreads();
-  constexpr int RC = CPLX ? 2 : 1;  // residue columns per D entry
-  for (int64_t n = blockIdx.x; n < P.cols; n += gridDim.x) {
-    const int ce = P.colexp[CPLX ? 2 * n : n];
-    if (ce >= kNonFiniteExp) continue;  // flagged column: the fix-up's
-    const int64_t dno = P.dn[n];
-    for (int64_t m0 = 4 * (int64_t)threadIdx.x; m0 < P.rows; m0 += 4 * (int64_t)blockDim.x) {
-      uint32_t w[RC][kMaxModuli];
+    double a[G], b[G], c[G];
 #pragma unroll
-      for (int j = 0; j < RC; ++j) crt_load4(P, n * RC + j, m0, w[j]);
+    for (int j = 0; j < G; ++j) a[j] = b[j] = c[j] = 0.0;
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int64_t m = m0 + t;
-        if (m >= P.rows) break;
-        const int re = P.rowexp[m];
-        if (re >= kNonFiniteExp) continue;  // flagged row: the fix-up's
-        const int e = re + ce - P.shift;
-        const int64_t o = P.dm[m] + dno;
-        uint32_t r[kMaxModuli];
-        crt_byte(w[0], t, r);
-        if constexpr (!CPLX) {
-          double* D = (double*)P.D;
-          const double v = P.ar * scale2(crt_combine(P, tab, r), e);
-          D[o] = P.br == 0.0 ? v : fma(P.br, D[o], v);
-        } else {
-          const double xr = scale2(crt_combine(P, tab, r), e);
-          crt_byte(w[RC - 1], t, r);
-          const double xi = scale2(crt_combine(P, tab, r), e);
-          double2* D = (double2*)P.D;
-          double2 v;
-          v.x = P.ar * xr - P.ai * xi;
-          v.y = P.ar * xi + P.ai * xr;
-          if (P.br != 0.0 || P.bi != 0.0) {
-            const double2 d = D[o];
-            v.x += P.br * d.x - P.bi * d.y;
-            v.y += P.br * d.y + P.bi * d.x;
-          }
-          D[o] = v;
+    for (int i = 0; i < kMaxModuli; ++i) {
+      if (i >= P.n) break;
+      const double s1 = P.s1[i], s2 = P.s2[i], s3 = P.s3[i];
+#pragma unroll
+      for (int j = 0; j < G; ++j) {
+        const uint32_t q = g == 0 ? (j < 4 ? w[i].x : w[i].y) : (j < 4 ? w[i].z : w[i].w);
+        // r as a double: 2^52 + r by its bits, minus 2^52
+        const double r = __hiloint2double(0x43300000, (int)__byte_perm(q, 0u, 0x4440 + (j & 3))) - 4503599627370496.0;
+        a[j] = fma(r, s1, a[j]);
+        b[j] = fma(r, s2, b[j]);
+        c[j] = fma(r, s3, c[j]);
+      }
+    }
+    auto combine = [&](int j, int cexp) {
+      const double Q = rint(a[j] * P.invM);
+      const double x = fma(-Q, P.M1, a[j]), y = fma(-Q, P.M2, b[j]), z = fma(-Q, P.M3, c[j]);  // exact
+      const double t = x + y, yy = t - x;
+      const double err = (x - (t - yy)) + (y - yy);  // x + y = t + err exactly
+      return scale2(t + (err + z), re + cexp - P.shift);
+    };
+#pragma unroll
+    for (int j = 0; j < H; ++j) {
+      if (o[j] < 0) continue;
+      if constexpr (!CPLX) {
+        const double v = P.ar * combine(j, ce[j]);
+        D[o[j]] = P.br == 0.0 ? v : fma(P.br, old[j], v);
+      } else {
+        const double xr = combine(2 * j, ce[j]), xi = combine(2 * j + 1, ce[j]);
+        double2 v;
+        v.x = P.ar * xr - P.ai * xi;
+        v.y = P.ar * xi + P.ai * xr;
+        if (read_d) {
+          v.x += P.br * old[j].x - P.bi * old[j].y;
+          v.y += P.br * old[j].y + P.bi * old[j].x;
         }
+        D[o[j]] = v;
       }
     }
   }
