@@ -133,9 +133,9 @@ TB_HD constexpr int pow2_mod(int e, int m) {
   for (int i = 0; i < e; ++i) r = (2 * r) % m;
   return r;
 }
-// c_ij = 2^(16 j) mod m_i in the symmetric range [-(m-1)/2, m/2]
-TB_HD constexpr int residue_cdig(int i, int j) {
-  const int m = residue_modulus(i), c = pow2_mod(16 * j, m);
+// 2^e mod m_i in the symmetric range [-(m-1)/2, m/2]
+TB_HD constexpr int residue_cdig(int i, int e) {
+  const int m = residue_modulus(i), c = pow2_mod(e, m);
   return c > (m - 1) / 2 ? c - m : c;
 }
 
@@ -158,71 +158,65 @@ struct GatherParams {
                        // split modes set it to 2047 for rows with a NaN or an infinity)
   int slices;
   int lanes_on_k;      // 1: consecutive k are contiguous in the source
+  int vec;             // 1 (lanes_on_k): aligned 16-byte groups of k are contiguous and aligned in the source
   double isign;        // -1 conjugates the imaginary part
   ResidueSpec rs;      // residue modes: the moduli
 };
 
-// Residues of integers |X| <= 2^p (p <= 63) held exactly as doubles.  X is
-// split once into balanced 16-bit digits D_j (|D_j| <= 2^15; three digits
-// when p <= 47), so that for every modulus the residue is
-//   raw = sum_j D_j c_j   (c_j = 2^(16 j) mod m in the symmetric range, c_0 = 1),
-// exact in FP32 (|raw| <= 4 * 2^15 * 128 = 2^24), then r = raw - m rint(raw / m)
-// in [-m/2, m/2] -- exact, the quotient rounded by the 1.5 * 2^23 trick (right
-// since raw / m is never within 1/(2m) of a half integer for odd m, and the
-// product's error is far below that).  The low byte of r, read off the bit
-// pattern of r + 1.5 * 2^23, is r in signed 8 bits (for m = 256, r = 128 gives
-// -128, the same residue).  For m = 256 the residue is D_0's low byte.
-struct Digits16 { float d[4]; };
+// Residues of integers |X| <= 2^p (p <= 52).  X is split once into digits D_j of
+// weight w_j, so that for every modulus the residue is
+//   raw = sum_j D_j c_j   (c_j = w_j mod m in the symmetric range, c_0 = 1),
+// exact in FP32 (|raw| < 2^24), then r = raw - m rint(raw / m) in [-m/2, m/2] --
+// exact, the quotient rounded by the 1.5 * 2^23 trick (right since raw / m is
+// never within 1/(2m) of a half integer for odd m, and the product's error is
+// far below that).  The low byte of r, read off the bit pattern of r + 1.5 *
+// 2^23, is r in signed 8 bits (for m = 256, r = 128 gives -128, the same
+// residue).  For m = 256 the residue is D_0's low byte.
+//
+// The digits come without conversions, for two values at a time.  Adding 1.5 *
+// 2^52 + B to v rounds v to the nearest integer X (one rounding: the sum lies in
+// [2^52, 2^53)) and leaves X + B in the sum's low mantissa bits; a 16-bit field u
+// placed under the bit pattern of 1.5 * 2^23 (one byte permute) is the float 1.5
+// * 2^23 + u, and one subtraction removes it with the field's bias.
+//   NDIG = 3 (p <= 46): B = 2^15 (1 + 2^16 + 2^32), digits u_j - 2^15 of weight 2^(16 j).
+//   NDIG = 4: X = 2^24 H + L with H = rint(v / 2^24) (|H| <= 2^28) and L = rint
+//   of the exact remainder (|L| <= 2^23); L + 2^23 + 2^15 and H + 2^28 + 2^15 give
+//   digits of weight 1, 2^16, 2^24 and 2^40.
+TB_HD constexpr int digit_weight(int ndig, int j) { return ndig == 3 ? 16 * j : (j == 0 ? 0 : j == 1 ? 16 : j == 2 ? 24 : 40); }
 
-// NDIG = 3: the top digit is x2 itself (|x2| <= 2^15 + 1 for p <= 47);
-// NDIG = 4: x2 is split once more (|x3| <= 2^(p-48) + 1).
+__device__ __forceinline__ float field_lo(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x4B400000u, 0x7610)); }
+__device__ __forceinline__ float field_hi(uint32_t w) { return __uint_as_float(__byte_perm(w, 0x4B400000u, 0x7632)); }
+
+// Digits of two operand values: X = rint(x 2^(se + p + 1)) with sc = 2^(se + p +
+// 1), or 0 when that is not a double (rows of tiny values, scaled in two steps).
 template <int NDIG>
-__device__ __forceinline__ Digits16 digits16(double X) {
-  Digits16 g;
-  const double x1 = rint(X * (1.0 / 65536.0));
-  g.d[0] = (float)fma(-x1, 65536.0, X);
-  const double x2 = rint(x1 * (1.0 / 65536.0));
-  g.d[1] = (float)fma(-x2, 65536.0, x1);
-  if constexpr (NDIG > 3) {
-    const double x3 = rint(x2 * (1.0 / 65536.0));
-    g.d[2] = (float)fma(-x3, 65536.0, x2);
-    g.d[3] = (float)x3;
-  } else {
-    g.d[2] = (float)x2;
-    g.d[3] = 0.f;
-  }
-  return g;
-}
-
-// Three balanced 16-bit digits of X = rint(v), |v| <= 2^46, without
-// conversions: Y = v + (1.5 * 2^52 + B), B = 2^15 (1 + 2^16 + 2^32), rounds v
-// to the nearest integer (one rounding: Y lies in [2^52, 2^53)) and leaves
-// X + B in Y's low 48 mantissa bits.  Its 16-bit fields u_j (0 <= u_j < 2^16)
-// give X = sum_j (u_j - 2^15) 2^(16 j); a field placed under the bit pattern
-// of 1.5 * 2^23 (one byte permute) is the float 1.5 * 2^23 + u_j, and one
-// subtraction gives d_j = u_j - 2^15 exactly.
-__device__ __forceinline__ Digits16 digits16_rint(double v) {
-  constexpr double kMB = 6896139076927488.0;  // 1.5 * 2^52 + 2^15 + 2^31 + 2^47
-  constexpr float kBias = 12582912.0f + 32768.0f;
-  const double Y = v + kMB;
-  const uint32_t lo = (uint32_t)__double2loint(Y), hi = (uint32_t)__double2hiint(Y);
-  Digits16 g;
-  g.d[0] = __uint_as_float(__byte_perm(lo, 0x4B400000u, 0x7610)) - kBias;
-  g.d[1] = __uint_as_float(__byte_perm(lo, 0x4B400000u, 0x7632)) - kBias;
-  g.d[2] = __uint_as_float(__byte_perm(hi, 0x4B400000u, 0x7610)) - kBias;
-  g.d[3] = 0.f;
-  return g;
-}
-
-// Digits of one operand value x of a row with scale exponent se: X = rint(x
-// 2^(se + p + 1)) for NDIG = 3 (sc = 2^(se + p + 1) when that is a double,
-// else 0), floor of the same for NDIG = 4.  Both are integers with |X| <= 2^p.
-template <int NDIG>
-__device__ __forceinline__ Digits16 operand_digits(double x, int se, double sc, double pscale) {
+__device__ __forceinline__ void digits2(double x0, int se0, double sc0, double x1, int se1, double sc1, double pscale,
+                                        float2 (&d)[4]) {
+  constexpr float kM = 12582912.0f;  // 1.5 * 2^23
+  constexpr double kM52 = 6755399441055744.0;  // 1.5 * 2^52
   if constexpr (NDIG == 3) {
-    return digits16_rint(sc != 0.0 ? x * sc : scale2(x, se) * pscale);
+    constexpr double kB = kM52 + 140739635871744.0;  // + 2^15 + 2^31 + 2^47
+    const double y0 = sc0 != 0.0 ? fma(x0, sc0, kB) : fma(scale2(x0, se0), pscale, kB);
+    const double y1 = sc1 != 0.0 ? fma(x1, sc1, kB) : fma(scale2(x1, se1), pscale, kB);
+    const uint32_t l0 = (uint32_t)__double2loint(y0), h0 = (uint32_t)__double2hiint(y0);
+    const uint32_t l1 = (uint32_t)__double2loint(y1), h1 = (uint32_t)__double2hiint(y1);
+    const float2 bias = make_float2(-(kM + 32768.0f), -(kM + 32768.0f));
+    d[0] = __fadd2_rn(make_float2(field_lo(l0), field_lo(l1)), bias);
+    d[1] = __fadd2_rn(make_float2(field_hi(l0), field_hi(l1)), bias);
+    d[2] = __fadd2_rn(make_float2(field_lo(h0), field_lo(h1)), bias);
   } else {
-    return digits16<NDIG>(floor(scale2(x, se) * pscale));
+    constexpr double kBH = kM52 + 268468224.0, kBL = kM52 + 8421376.0;  // + 2^28 + 2^15; + 2^23 + 2^15
+    const double v0 = sc0 != 0.0 ? x0 * sc0 : scale2(x0, se0) * pscale, v1 = sc1 != 0.0 ? x1 * sc1 : scale2(x1, se1) * pscale;
+    const double h0 = fma(v0, 0x1p-24, kBH), h1 = fma(v1, 0x1p-24, kBH);
+    const double l0 = fma(kBH - h0, 0x1p24, v0) + kBL, l1 = fma(kBH - h1, 0x1p24, v1) + kBL;
+    const uint32_t wl0 = (uint32_t)__double2loint(l0), wl1 = (uint32_t)__double2loint(l1);
+    const uint32_t wh0 = (uint32_t)__double2loint(h0), wh1 = (uint32_t)__double2loint(h1);
+    const float2 b16 = make_float2(-(kM + 32768.0f), -(kM + 32768.0f)), b7 = make_float2(-(kM + 128.0f), -(kM + 128.0f)),
+                 b12 = make_float2(-(kM + 4096.0f), -(kM + 4096.0f));
+    d[0] = __fadd2_rn(make_float2(field_lo(wl0), field_lo(wl1)), b16);
+    d[1] = __fadd2_rn(make_float2(field_hi(wl0), field_hi(wl1)), b7);
+    d[2] = __fadd2_rn(make_float2(field_lo(wh0), field_lo(wh1)), b16);
+    d[3] = __fadd2_rn(make_float2(field_hi(wh0), field_hi(wh1)), b12);
   }
 }
 
@@ -238,7 +232,8 @@ __device__ __forceinline__ float2 residue_shifted2(const float2 (&d)[4]) {
     return __fadd2_rn(d[0], magic);
   } else {
     constexpr float negm = -(float)m, inv = 1.0f / (float)m;
-    constexpr float c1 = (float)residue_cdig(I, 1), c2 = (float)residue_cdig(I, 2), c3 = (float)residue_cdig(I, 3);
+    constexpr float c1 = (float)residue_cdig(I, digit_weight(NDIG, 1)), c2 = (float)residue_cdig(I, digit_weight(NDIG, 2)),
+                    c3 = (float)residue_cdig(I, digit_weight(NDIG, NDIG > 3 ? 3 : 2));
     float2 raw = __ffma2_rn(d[1], make_float2(c1, c1), d[0]);
     raw = __ffma2_rn(d[2], make_float2(c2, c2), raw);
     if constexpr (NDIG > 3) raw = __ffma2_rn(d[3], make_float2(c3, c3), raw);
@@ -254,15 +249,9 @@ __device__ __forceinline__ uint32_t pack_low_bytes(float a, float b, float c, fl
   return __byte_perm(lo, hi, 0x5410);
 }
 
-// Residue I of four values, packed little-endian.
+// Residue I of four values (two pairs), packed little-endian.
 template <int NDIG, int I>
-__device__ __forceinline__ uint32_t residue4(const Digits16 (&g)[4]) {
-  float2 a[4], b[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    a[j] = make_float2(g[0].d[j], g[1].d[j]);
-    b[j] = make_float2(g[2].d[j], g[3].d[j]);
-  }
+__device__ __forceinline__ uint32_t residue4(const float2 (&a)[4], const float2 (&b)[4]) {
   const float2 ra = residue_shifted2<NDIG, I>(a), rb = residue_shifted2<NDIG, I>(b);
   return pack_low_bytes(ra.x, ra.y, rb.x, rb.y);
 }
@@ -307,17 +296,30 @@ struct GatherElem {
   using R = typename std::conditional<F32, float, double>::type;
   using E = typename std::conditional<CPLX, typename std::conditional<F32, float2, double2>::type, R>::type;
 };
+// Tile of a gather mode: TM rows x TK contracted values in two buffers, rows of
+// CH 16-byte chunks and one chunk of padding.  A conversion thread takes KPT
+// consecutive k of a row (G chunks); chunk c of a row sits at c ^ ((c / G) & 7),
+// so that the eight threads of a quarter warp read eight different 16-byte
+// banks, and copies along k or along rows write without conflicts beyond two.
+template <int MODE>
+struct GatherTile {
+  using E = typename GatherElem<MODE>::E;
+  static constexpr int ES = (int)sizeof(E), TM = gather_rows<E>(), TK = kGK;
+  static constexpr int KPT = MODE == G_RESID_R8 || MODE == G_SPLIT_R4 ? 8 : 4;
+  static constexpr int G = KPT * ES / 16, CH = TK * ES / 16, PITCH = (CH + 1) * 16;
+  static constexpr int BUF = TM * PITCH;
+  static __device__ __forceinline__ int chunk(int c) { return (c ^ ((c / G) & 7)) * 16; }
+  static __device__ __forceinline__ int at(int k) {
+    const int byte = k * ES;
+    return chunk(byte >> 4) + (byte & 15);
+  }
+};
 // Dynamic shared memory of a gather CTA: two tile buffers, a ring of three
 // tiles' K offsets, the row offsets and the row scale exponents.
-// K tile of a gather mode (64 for all: 32-wide tiles with four CTAs per SM
-// ran the real residue gather 1.7x slower)
-template <int MODE>
-constexpr int gather_tk() { return kGK; }
 template <int MODE>
 constexpr int gather_smem_bytes() {
-  using E = typename GatherElem<MODE>::E;
-  return 2 * gather_rows<E>() * (gather_tk<MODE>() + 1) * (int)sizeof(E) + 3 * gather_tk<MODE>() * 8 +
-         gather_rows<E>() * 20;
+  using T = GatherTile<MODE>;
+  return 2 * T::BUF + 3 * T::TK * 8 + T::TM * 20;
 }
 
 // Asynchronous copy of one element into shared memory; zero-filled when
@@ -332,31 +334,28 @@ __device__ __forceinline__ void cp_async_elem(void* sdst, const void* gsrc, bool
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(gsrc), "n"(BYTES), "r"(n) : "memory");
 }
 
+// Bound by instruction issue, not by HBM: the conversion costs about 5 packed
+// instructions per value pair and modulus.  A thread's copies therefore share
+// one row or one k (a table read and an addition per copy, or one 16-byte copy
+// per two or four values where `vec` allows), and its conversions share the
+// digits of eight values and store 8 bytes per plane.
 template <int MODE, int NDIG = 3>
 __device__ __forceinline__ void gather_body(const GatherParams& P, int64_t rowtile, int ky, int kstep) {
   constexpr bool CPLX = GatherElem<MODE>::CPLX;
   constexpr bool F32 = GatherElem<MODE>::F32;
-  using R = typename GatherElem<MODE>::R;
   using E = typename GatherElem<MODE>::E;
-  (void)sizeof(R);
-  constexpr int TM = gather_rows<E>(), TK = gather_tk<MODE>();
+  using T = GatherTile<MODE>;
+  constexpr int TM = T::TM, TK = T::TK, ES = T::ES, KPT = T::KPT;
   // Tiles move global -> shared with cp.async, double-buffered: tile i+1 is in
   // flight while tile i converts, without passing through registers.  Its
   // source addresses need the K offsets of tile i+1, which sit in shared
   // memory: they were read from global memory (into a register, by one thread
   // per k) during tile i-1's conversion and stored at its end.
   extern __shared__ __align__(16) unsigned char gather_smem[];
-  E* tbuf = reinterpret_cast<E*>(gather_smem);                                        // [2][TM][TK+1]
-  int64_t* lkbuf = reinterpret_cast<int64_t*>(gather_smem + 2 * TM * (TK + 1) * sizeof(E));  // [3][TK]
-  int64_t* sm_lm = lkbuf + 3 * TK;                                                     // [TM]
+  int64_t* lkbuf = reinterpret_cast<int64_t*>(gather_smem + 2 * T::BUF);  // [3][TK]
+  int64_t* sm_lm = lkbuf + 3 * TK;                                         // [TM]
   double* sm_sc = reinterpret_cast<double*>(sm_lm + TM);  // residue modes: 2^(se + p + 1), or 0
   int* sm_se = reinterpret_cast<int*>(sm_sc + TM);  // slice and residue modes: the row's scale exponent
-  auto tile_at = [&](int b) { return reinterpret_cast<E (*)[TK + 1]>(tbuf + (size_t)b * TM * (TK + 1)); };
-  // Within a row, k sits at column (k % 4) * TK/4 + k / 4: the conversion's
-  // lanes read k = 4j + t for the TK/4 lanes j of a row, which then fall on
-  // consecutive columns (no bank conflicts within a row) instead of every
-  // fourth one.
-  auto col = [](int k) { return (k & 3) * (TK / 4) + (k >> 2); };
   const int64_t m0 = rowtile * TM;
   const int tid = threadIdx.x;
   const E* src = (const E*)P.src;
@@ -376,16 +375,46 @@ __device__ __forceinline__ void gather_body(const GatherParams& P, int64_t rowti
       lkbuf[j * TK + tid] = k < P.K ? P.lk[k] : 0;
     }
   }
-  constexpr int IT = TM * TK / kGThreads;
-  auto issue_tile = [&](int64_t k0, int b, const int64_t* lkt) {
-    E (*t)[TK + 1] = tile_at(b);
+  auto issue_tile = [&](int64_t k0, int buf, const int64_t* lkt) {
+    unsigned char* t = gather_smem + (size_t)buf * T::BUF;
+    const int64_t kleft = P.K - k0;
+    if (P.lanes_on_k && (P.vec || ES == 16)) {
+      constexpr int VW = 16 / ES, RS = kGThreads / T::CH;  // values per copy, rows per round
+      static_assert(kGThreads % T::CH == 0 && TM % RS == 0, "whole rounds");
+      const int ch = tid % T::CH, r0 = tid / T::CH;
+      const bool kv = ch * VW < kleft;
+      const E* base = src + (kv ? lkt[ch * VW] : 0);
+      unsigned char* d = t + r0 * T::PITCH + T::chunk(ch);
 #pragma unroll
-    for (int it = 0; it < IT; ++it) {
-      const int idx = tid + it * kGThreads;
-      const int mm = P.lanes_on_k ? idx / TK : idx % TM;
-      const int kk = P.lanes_on_k ? idx % TK : idx / TM;
-      const bool valid = sm_lm[mm] >= 0 && k0 + kk < P.K;
-      cp_async_elem<(int)sizeof(E)>(&t[mm][col(kk)], valid ? src + sm_lm[mm] + lkt[kk] : src, valid);
+      for (int it = 0; it < TM / RS; ++it) {
+        const int64_t lm = sm_lm[r0 + it * RS];
+        const bool ok = kv && lm >= 0;
+        cp_async_elem<16>(d + it * RS * T::PITCH, base + (ok ? lm : 0), ok);
+      }
+    } else if (P.lanes_on_k) {
+      constexpr int RS = kGThreads / TK;
+      const int kk = tid % TK, r0 = tid / TK;
+      const bool kv = kk < kleft;
+      const E* base = src + (kv ? lkt[kk] : 0);
+      unsigned char* d = t + r0 * T::PITCH + T::at(kk);
+#pragma unroll
+      for (int it = 0; it < TM / RS; ++it) {
+        const int64_t lm = sm_lm[r0 + it * RS];
+        const bool ok = kv && lm >= 0;
+        cp_async_elem<ES>(d + it * RS * T::PITCH, base + (ok ? lm : 0), ok);
+      }
+    } else {
+      constexpr int KS = kGThreads / TM;
+      const int r = tid % TM, kk0 = tid / TM;
+      const int64_t lm = sm_lm[r];
+      const E* base = src + (lm >= 0 ? lm : 0);
+      unsigned char* d = t + r * T::PITCH;
+#pragma unroll
+      for (int it = 0; it < TK / KS; ++it) {
+        const int kk = kk0 + it * KS;
+        const bool ok = lm >= 0 && kk < kleft;
+        cp_async_elem<ES>(d + T::at(kk), base + (ok ? lkt[kk] : 0), ok);
+      }
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
@@ -406,69 +435,67 @@ __device__ __forceinline__ void gather_body(const GatherParams& P, int64_t rowti
     }
     asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // this thread's copies of tile i
     __syncthreads();                                          // everyone's
-    E (*tile)[TK + 1] = tile_at(i & 1);
+    const unsigned char* tile = gather_smem + (size_t)(i & 1) * T::BUF;
     {
-      // convert: thread -> (row mm, 4 consecutive k)
-      for (int idx = tid; idx < TM * (TK / 4); idx += kGThreads) {
-        const int mm = idx / (TK / 4), kq = (idx % (TK / 4)) * 4;
+      // convert: thread -> (row mm, KPT consecutive k)
+      for (int idx = tid; idx < TM * (TK / KPT); idx += kGThreads) {
+        const int mm = idx / (TK / KPT), kj = idx % (TK / KPT), kq = kj * KPT;
         const int64_t m = m0 + mm, k = k0 + kq;
+        union { uint4 q[T::G]; E v[KPT]; } in;
+#pragma unroll
+        for (int u = 0; u < T::G; ++u)
+          in.q[u] = *reinterpret_cast<const uint4*>(tile + mm * T::PITCH + (((kj * T::G + u) ^ (kj & 7)) * 16));
         if constexpr (MODE == G_RESID_R8) {
           const int se = sm_se[mm];
           const double sc = sm_sc[mm];
-          Digits16 g[4];
+          float2 g[4][4];
 #pragma unroll
-          for (int t = 0; t < 4; ++t) g[t] = operand_digits<NDIG>(tile[mm][col(kq + t)], se, sc, P.rs.pscale);
+          for (int t = 0; t < 4; ++t) digits2<NDIG>(in.v[2 * t], se, sc, in.v[2 * t + 1], se, sc, P.rs.pscale, g[t]);
           int8_t* base = (int8_t*)P.planes + m * P.kpad + k;
           for_moduli<0, kMaxModuli>(P.rs.n, [&](auto ic) {
             constexpr int I = decltype(ic)::value;
-            *reinterpret_cast<uint32_t*>(base + I * P.pstride) = residue4<NDIG, I>(g);
+            *reinterpret_cast<uint2*>(base) = make_uint2(residue4<NDIG, I>(g[0], g[1]), residue4<NDIG, I>(g[2], g[3]));
+            base += P.pstride;
           });
         } else if constexpr (MODE == G_RESID_C8A) {
           // A' row m: (re, im) interleaved along K
           const int se = sm_se[mm];
           const double sc = sm_sc[mm];
-          Digits16 ga[4], gb[4];
+          float2 g[4][4];
 #pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const E v0 = tile[mm][col(kq + t)], v1 = tile[mm][col(kq + 2 + t)];
-            ga[2 * t] = operand_digits<NDIG>(v0.x, se, sc, P.rs.pscale);
-            ga[2 * t + 1] = operand_digits<NDIG>(P.isign * v0.y, se, sc, P.rs.pscale);
-            gb[2 * t] = operand_digits<NDIG>(v1.x, se, sc, P.rs.pscale);
-            gb[2 * t + 1] = operand_digits<NDIG>(P.isign * v1.y, se, sc, P.rs.pscale);
-          }
+          for (int t = 0; t < 4; ++t)
+            digits2<NDIG>(in.v[t].x, se, sc, P.isign * in.v[t].y, se, sc, P.rs.pscale, g[t]);
           int8_t* base = (int8_t*)P.planes + m * P.kpad + 2 * k;
           for_moduli<0, kMaxModuli>(P.rs.n, [&](auto ic) {
             constexpr int I = decltype(ic)::value;
-            *reinterpret_cast<uint2*>(base + I * P.pstride) = make_uint2(residue4<NDIG, I>(ga), residue4<NDIG, I>(gb));
+            *reinterpret_cast<uint2*>(base) = make_uint2(residue4<NDIG, I>(g[0], g[1]), residue4<NDIG, I>(g[2], g[3]));
+            base += P.pstride;
           });
         } else if constexpr (MODE == G_RESID_C8B) {
-          // B' rows 2n = (re, -im), 2n+1 = (im, re) interleaved along K
+          // B' rows 2n = (re, -im), 2n+1 = (im, re) interleaved along K; the
+          // residues of -im are those of im, negated byte by byte
           const int se = sm_se[mm];
           const double sc = sm_sc[mm];
-          Digits16 R[4], I[4], NI[4];
+          float2 R[2][4], I[2][4];
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const E v = tile[mm][col(kq + t)];
-            R[t] = operand_digits<NDIG>(v.x, se, sc, P.rs.pscale);
-            I[t] = operand_digits<NDIG>(P.isign * v.y, se, sc, P.rs.pscale);
-            NI[t] = operand_digits<NDIG>(-P.isign * v.y, se, sc, P.rs.pscale);
+          for (int t = 0; t < 2; ++t) {
+            digits2<NDIG>(in.v[2 * t].x, se, sc, in.v[2 * t + 1].x, se, sc, P.rs.pscale, R[t]);
+            digits2<NDIG>(P.isign * in.v[2 * t].y, se, sc, P.isign * in.v[2 * t + 1].y, se, sc, P.rs.pscale, I[t]);
           }
-          const Digits16 r0a[4] = {R[0], NI[0], R[1], NI[1]}, r0b[4] = {R[2], NI[2], R[3], NI[3]};
-          const Digits16 r1a[4] = {I[0], R[0], I[1], R[1]}, r1b[4] = {I[2], R[2], I[3], R[3]};
           int8_t* b0 = (int8_t*)P.planes + (2 * m) * P.kpad + 2 * k;
-          int8_t* b1 = b0 + P.kpad;
           for_moduli<0, kMaxModuli>(P.rs.n, [&](auto ic) {
             constexpr int J = decltype(ic)::value;
-            *reinterpret_cast<uint2*>(b0 + J * P.pstride) =
-                make_uint2(residue4<NDIG, J>(r0a), residue4<NDIG, J>(r0b));
-            *reinterpret_cast<uint2*>(b1 + J * P.pstride) =
-                make_uint2(residue4<NDIG, J>(r1a), residue4<NDIG, J>(r1b));
+            const uint32_t re = residue4<NDIG, J>(R[0], R[1]), im = residue4<NDIG, J>(I[0], I[1]);
+            const uint32_t ni = __vsub4(0u, im);
+            *reinterpret_cast<uint2*>(b0) = make_uint2(__byte_perm(re, ni, 0x5140), __byte_perm(re, ni, 0x7362));
+            *reinterpret_cast<uint2*>(b0 + P.kpad) = make_uint2(__byte_perm(im, re, 0x5140), __byte_perm(im, re, 0x7362));
+            b0 += P.pstride;
           });
         } else if constexpr (MODE == G_SLICE_R8) {
           const int se = sm_se[mm];
           long long X[4];
 #pragma unroll
-          for (int t = 0; t < 4; ++t) X[t] = fixed55(scale2(tile[mm][col(kq + t)], se));
+          for (int t = 0; t < 4; ++t) X[t] = fixed55(scale2(in.v[t], se));
           int8_t* base = (int8_t*)P.planes + m * P.kpad + k;
 #pragma unroll
           for (int i = 0; i < kMaxSlicesDev; ++i)
@@ -479,7 +506,7 @@ __device__ __forceinline__ void gather_body(const GatherParams& P, int64_t rowti
           long long R[4], I[4];
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
-            const E v = tile[mm][col(kq + t)];
+            const E v = in.v[t];
             R[t] = fixed55(scale2(v.x, se));
             I[t] = fixed55(scale2(P.isign * v.y, se));
           }
@@ -496,7 +523,7 @@ __device__ __forceinline__ void gather_body(const GatherParams& P, int64_t rowti
           long long R[4], I[4], NI[4];
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
-            const E v = tile[mm][col(kq + t)];
+            const E v = in.v[t];
             const double im = scale2(P.isign * v.y, se);
             R[t] = fixed55(scale2(v.x, se));
             I[t] = fixed55(im);
@@ -513,25 +540,26 @@ __device__ __forceinline__ void gather_body(const GatherParams& P, int64_t rowti
                   make_uint2(slice4(I[0], R[0], I[1], R[1], i), slice4(I[2], R[2], I[3], R[3], i));
             }
         } else if constexpr (MODE == G_SPLIT_R4) {
-          __nv_bfloat16 h[4], l[4];
+          __nv_bfloat16 h[8], l[8];
           bool nf = false;
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            split_bf16(tile[mm][col(kq + t)], h[t], l[t]);
-            nf |= !isfinite(tile[mm][col(kq + t)]);
+          for (int t = 0; t < 8; ++t) {
+            split_bf16(in.v[t], h[t], l[t]);
+            nf |= !isfinite(in.v[t]);
           }
           if (nf && P.rowE && m < P.rows) atomicMax(&P.rowE[m], 2047u);  // row left to the non-finite fix-up
           __nv_bfloat16* base = (__nv_bfloat16*)P.planes + m * P.kpad + k;
-          __nv_bfloat162 hh[2] = {{h[0], h[1]}, {h[2], h[3]}}, ll[2] = {{l[0], l[1]}, {l[2], l[3]}};
-          *reinterpret_cast<uint2*>(base) = *reinterpret_cast<uint2*>(hh);
-          *reinterpret_cast<uint2*>(base + P.pstride) = *reinterpret_cast<uint2*>(ll);
+          __nv_bfloat162 hh[4] = {{h[0], h[1]}, {h[2], h[3]}, {h[4], h[5]}, {h[6], h[7]}};
+          __nv_bfloat162 ll[4] = {{l[0], l[1]}, {l[2], l[3]}, {l[4], l[5]}, {l[6], l[7]}};
+          *reinterpret_cast<uint4*>(base) = *reinterpret_cast<uint4*>(hh);
+          *reinterpret_cast<uint4*>(base + P.pstride) = *reinterpret_cast<uint4*>(ll);
         } else {
           // complex FP32: A' rows (re, im); B' rows 2n (re, -im), 2n+1 (im, re)
           __nv_bfloat16 hr[4], lr[4], hi[4], li[4], nhi[4], nli[4];
           bool nf = false;
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
-            const E v = tile[mm][col(kq + t)];
+            const E v = in.v[t];
             const float im = (float)P.isign * v.y;
             split_bf16(v.x, hr[t], lr[t]);
             split_bf16(im, hi[t], li[t]);
