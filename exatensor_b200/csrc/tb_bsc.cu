@@ -493,6 +493,13 @@ int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t*
       G.rowE = pl->rowE + o.e_off;
       G.slices = pl->slices;
       G.lanes_on_k = (o.ks[0].s1 == 1 || o.rows[0].s1 != 1) ? 1 : 0;
+      {  // 16-byte copies: whole groups of k that are contiguous and aligned in the block
+        const int64_t vw = pl->i8 ? 2 : 4;
+        bool vec = o.ks[0].s1 == 1 && o.ks[0].ext % vw == 0 && (uintptr_t)o.ptr % 16 == 0;
+        for (size_t i = 1; i < o.ks.size(); ++i) vec = vec && o.ks[i].s1 % vw == 0;
+        for (auto& g : o.rows) vec = vec && g.s1 % vw == 0;
+        G.vec = vec ? 1 : 0;
+      }
       G.isign = 1.0;
       const int job = (int)jobs.size();
       jobs.push_back(G);

@@ -232,12 +232,33 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
   (void)ddims;
   if (Z0.K < 1 || Z0.M < 1 || Z0.N < 1 || Z0.k.empty()) return TB_ERR_NOT_IMPLEMENTED;
   Matricization Z = Z0;
-  // rows in D-stride order so that consecutive epilogue lanes write consecutive D
+  // unit extents carry no index; rows in D-stride order so that consecutive
+  // epilogue lanes write consecutive D
   auto by_d = [](const MGroup& x, const MGroup& y) { return x.s2 < y.s2; };
+  auto no_units = [](std::vector<MGroup>& g) {
+    g.erase(std::remove_if(g.begin(), g.end(), [](const MGroup& x) { return x.ext == 1; }), g.end());
+  };
+  auto unit_of = [](const std::vector<MGroup>& g, bool second) {
+    for (size_t i = 0; i < g.size(); ++i)
+      if ((second ? g[i].s2 : g[i].s1) == 1) return (int)i;
+    return -1;
+  };
+  no_units(Z.m);
+  no_units(Z.n);
+  no_units(Z.k);
   std::stable_sort(Z.m.begin(), Z.m.end(), by_d);
   std::stable_sort(Z.n.begin(), Z.n.end(), by_d);
   // the operand holding D's fastest dimension plays the row (M) role
   const bool swap = !Z.n.empty() && (Z.m.empty() || Z.n[0].s2 < Z.m[0].s2);
+  // contracted order: an index that is contiguous in an operand comes first (the
+  // larger operand's where both have one), so that its gather runs along it
+  {
+    const int kl = unit_of(Z.k, false), kr = unit_of(Z.k, true);
+    const bool by_r = kl < 0 || (kr >= 0 && Z.N > Z.M);
+    std::stable_sort(Z.k.begin(), Z.k.end(), [&](const MGroup& x, const MGroup& y) {
+      return by_r && kr >= 0 ? x.s2 < y.s2 : x.s1 < y.s1;
+    });
+  }
   Operand Lop{l, Z.m, {}, lconj != 0}, Rop{r, Z.n, {}, rconj != 0};
   for (auto g : Z.k) {
     Lop.ks.push_back(g);                       // s1 = L stride
@@ -245,7 +266,10 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
   }
   (void)ldims; (void)rdims;
   const Operand& A = swap ? Rop : Lop;
-  const Operand& B = swap ? Lop : Rop;
+  Operand& B = swap ? Lop : Rop;
+  // columns: the operand's contiguous group first (a column's place among the
+  // others matters to no write of D)
+  if (const int u = unit_of(B.rows, false); u > 0) std::rotate(B.rows.begin(), B.rows.begin() + u, B.rows.begin() + u + 1);
   const bool cplx = is_complex(dtk), i8 = is_double(dtk);
   int64_t M = 1, Nc = 1;
   for (auto& g : A.rows) M *= g.ext;
@@ -361,8 +385,8 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
   const size_t offA = 0, offB = al(bytesA), offDm = offB + al(bytesB), offDn = offDm + al(M * 8),
                offLA = offDn + al(Nc * 8), offLB = offLA + al(M * 8), offKA = offLB + al(Nc * 8),
                offKB = offKA + al(K * 8), offRE = offKB + al(K * 8), offCE = offRE + al(M * 4),
-               offRX = offCE + al(Nc * 4), offCX = offRX + al(M * 4), offBR = offCX + al(Nr * 4),
-               offBC = offBR + al(M * 4), offNB = offBC + al(Nc * 4), offRES = offNB + 256,
+               offNB = offCE + al(Nc * 4), offRX = offNB + 256, offCX = offRX + al(M * 4), offBR = offCX + al(Nr * 4),
+               offBC = offBR + al(M * 4), offRES = offBC + al(Nc * 4),
                total = offRES + (resid ? al((size_t)RP.rs.n * Npad * Mpad) : 0);
   unsigned char* ws = nullptr;
   if (int e = scratch_alloc((void**)&ws, total, s)) return e;
@@ -384,69 +408,71 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
   int* nbad = (int*)(ws + offNB);
   const int64_t ksrc_pad = cplx ? Kpad / 2 : Kpad;  // padded K in source elements
   do {
-    if ((err = build_offsets(A.rows, true, dm, s))) break;
-    if ((err = build_offsets(B.rows, true, dn, s))) break;
-    if ((err = build_offsets(A.rows, false, lmA, s))) break;
-    if ((err = build_offsets(B.rows, false, lmB, s))) break;
-    if ((err = build_offsets(A.ks, false, lkA, s))) break;
-    if ((err = build_offsets(B.ks, false, lkB, s))) break;
+    // Offset tables and cleared words (row maxima, counters) in one launch.  A's
+    // rows run in blocks of its contiguous group where that is not D's fastest
+    // one: the gathers then read 64 bytes at a time instead of single elements
+    // (40^6 R8: row maxima and gathers 132 -> 60 us).  The residue path's
+    // reconstruction steps over the blocks; the epilogues that write D directly
+    // write runs of four instead, once per accumulator pass, so they take blocks
+    // only where the operand's bytes outweigh that.
+    const int pa = !A.ks.empty() && A.ks[0].s1 == 1 ? -1 : unit_of(A.rows, false);
+    const bool blocked = pa > 0 && (resid || 32.0 * (double)K > 8.0 * (double)Nr * (double)passes.size());
+    const int kRowBlock = 8;
+    TableParams TP;
+    std::memset(&TP, 0, sizeof(TP));
+    if (blocked) set_blocked_job(&TP.job[0], A.rows, pa, kRowBlock, lmA, dm);
+    else set_table_job(&TP.job[0], A.rows, lmA, dm);
+    set_table_job(&TP.job[1], B.rows, lmB, dn);
+    {
+      std::vector<MGroup> ks = A.ks;  // s1: A's stride, s2: B's
+      for (size_t i = 0; i < ks.size(); ++i) ks[i].s2 = B.ks[i].s1;
+      set_table_job(&TP.job[2], ks, lkA, lkB);
+    }
+    TP.zero = (uint32_t*)rowE;
+    TP.zero_words = (int64_t)(offRX - offRE) / 4;
+    if ((err = run_tables(TP, s))) break;
     GatherParams GA{}, GB{};
     GA.src = A.ptr; GA.lm = lmA; GA.lk = lkA; GA.rows = M; GA.K = K; GA.kpad = Kpad; GA.pstride = Mpad * Kpad;
     GA.planes = Ap; GA.rowE = rowE; GA.slices = S; GA.isign = A.conj ? -1.0 : 1.0;
-    GA.lanes_on_k = (A.ks[0].s1 == 1 || A.rows.empty() || A.rows[0].s1 != 1) ? 1 : 0;
+    // 16-byte copies: whole groups of k that are contiguous and aligned in the operand
+    auto lanes = [&](GatherParams& G, const Operand& O, bool rows_run) {
+      const int64_t vw = 16 / elem_bytes(dtk);
+      G.lanes_on_k = (!O.ks.empty() && O.ks[0].s1 == 1) || !rows_run ? 1 : 0;
+      bool vec = !O.ks.empty() && O.ks[0].s1 == 1 && O.ks[0].ext % vw == 0 && (uintptr_t)O.ptr % 16 == 0;
+      for (size_t i = 1; i < O.ks.size(); ++i) vec = vec && O.ks[i].s1 % vw == 0;
+      for (auto& g : O.rows) vec = vec && g.s1 % vw == 0;
+      G.vec = vec ? 1 : 0;
+    };
+    lanes(GA, A, blocked || pa == 0);
     if (resid) GA.rs = RP.rs;
     GB.src = B.ptr; GB.lm = lmB; GB.lk = lkB; GB.rows = Nc; GB.K = K; GB.kpad = Kpad; GB.pstride = Npad * Kpad;
     GB.planes = Bp; GB.rowE = colE; GB.slices = S; GB.isign = B.conj ? -1.0 : 1.0;
-    GB.lanes_on_k = (B.ks[0].s1 == 1 || B.rows.empty() || B.rows[0].s1 != 1) ? 1 : 0;
+    lanes(GB, B, !B.rows.empty() && B.rows[0].s1 == 1);
     if (resid) GB.rs = RP.rs;
     const int tmr = i8 && cplx ? 32 : 64;               // gather tile rows (16-byte elements: 32)
     const int64_t gA = Mpad / tmr, gB = (cplx ? Npad / 2 : Npad) / tmr, gk = ksrc_pad / kGK;
     // row / column exponents and the lists of rows and columns flagged as
     // holding a NaN or an infinity (exponent field 2047): the epilogue leaves
-    // their D entries to nonfinite_fixup_kernel
-    if (cudaMemsetAsync(rowE, 0, offRX - offRE, s) != cudaSuccess) { err = TB_ERR_CUDA; break; }
-    // nbad[0..1]: flagged row / column counts; nbad[2]: the GEMM's work-unit counter
-    if (cudaMemsetAsync(nbad, 0, 4 * sizeof(int), s) != cudaSuccess) { err = TB_ERR_CUDA; break; }
+    // their D entries to nonfinite_fixup_kernel.  nbad[0..1]: flagged row /
+    // column counts; nbad[2]: the GEMM's work-unit counter.
     auto run_exps = [&]() -> int {
-      exps_kernel<<<std::max<int64_t>(1, std::min<int64_t>((M + 255) / 256, 4096)), 256, 0, s>>>(rowE, rowx, M, 1,
-                                                                                                 badrows, nbad);
-      TB_CHECK_LAUNCH();
-      exps_kernel<<<std::max<int64_t>(1, std::min<int64_t>((Nr + 255) / 256, 4096)), 256, 0, s>>>(
-          colE, colx, Nr, cplx ? 2 : 1, badcols, nbad + 1);
+      exps_pair_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((M + Nr + 255) / 256, 4096)), 256, 0, s>>>(
+          rowE, rowx, M, badrows, colE, colx, Nr, cplx ? 2 : 1, badcols, nbad);
       TB_CHECK_LAUNCH();
       return 0;
     };
     if (i8) {
-      const int64_t eA = (M + tmr - 1) / tmr, eB = (Nc + tmr - 1) / tmr, ek = (K + kGK - 1) / kGK;
-      if (!cplx) {
-        if ((err = run_rowmax<false>(GA, eA, ek, s))) break;
-        if ((err = run_rowmax<false>(GB, eB, ek, s))) break;
-      } else {
-        if ((err = run_rowmax<true>(GA, eA, ek, s))) break;
-        if ((err = run_rowmax<true>(GB, eB, ek, s))) break;
-      }
+      if ((err = cplx ? run_rowmax<true>(GA, GB, s) : run_rowmax<false>(GA, GB, s))) break;
       if ((err = run_exps())) break;
-      if (resid && !cplx) {
-        if ((err = run_gather<G_RESID_R8>(GA, gA, gk, s))) break;
-        if ((err = run_gather<G_RESID_R8>(GB, gB, gk, s))) break;
-      } else if (resid) {
-        if ((err = run_gather<G_RESID_C8A>(GA, gA, gk, s))) break;
-        if ((err = run_gather<G_RESID_C8B>(GB, gB, gk, s))) break;
-      } else if (!cplx) {
-        if ((err = run_gather<G_SLICE_R8>(GA, gA, gk, s))) break;
-        if ((err = run_gather<G_SLICE_R8>(GB, gB, gk, s))) break;
-      } else {
-        if ((err = run_gather<G_SLICE_C8A>(GA, gA, gk, s))) break;
-        if ((err = run_gather<G_SLICE_C8B>(GB, gB, gk, s))) break;
-      }
+      if (resid) err = cplx ? run_gather<G_RESID_C8A, G_RESID_C8B>(GA, GB, gA, gB, gk, s)
+                            : run_gather<G_RESID_R8, G_RESID_R8>(GA, GB, gA, gB, gk, s);
+      else err = cplx ? run_gather<G_SLICE_C8A, G_SLICE_C8B>(GA, GB, gA, gB, gk, s)
+                      : run_gather<G_SLICE_R8, G_SLICE_R8>(GA, GB, gA, gB, gk, s);
+      if (err) break;
     } else {
-      if (!cplx) {
-        if ((err = run_gather<G_SPLIT_R4>(GA, gA, gk, s))) break;
-        if ((err = run_gather<G_SPLIT_R4>(GB, gB, gk, s))) break;
-      } else {
-        if ((err = run_gather<G_SPLIT_C4A>(GA, gA, gk, s))) break;
-        if ((err = run_gather<G_SPLIT_C4B>(GB, gB, gk, s))) break;
-      }
+      if ((err = cplx ? run_gather<G_SPLIT_C4A, G_SPLIT_C4B>(GA, GB, gA, gB, gk, s)
+                      : run_gather<G_SPLIT_R4, G_SPLIT_R4>(GA, GB, gA, gB, gk, s)))
+        break;
       if ((err = run_exps())) break;  // the split gathers flag non-finite rows
     }
     // GEMM parameters
@@ -509,7 +535,9 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
       C.dm = dm; C.dn = dn; C.D = d;
       C.rowexp = rowx; C.colexp = colx;
       C.ar = realpha; C.ai = cplx ? ai : 0.0; C.br = P.br; C.bi = 0.0;
-      const int64_t rb = (M + 31) / 32, cb = (Nr + kCrtCols * kCrtWarps - 1) / (kCrtCols * kCrtWarps);
+      C.row_step = blocked ? kRowBlock : 1;
+      const int64_t rb = (M + 32 * C.row_step - 1) / (32 * C.row_step) * C.row_step,
+                    cb = (Nr + kCrtCols * kCrtWarps - 1) / (kCrtCols * kCrtWarps);
       if (rb * cb > INT32_MAX) { set_error("residue reconstruction grid too large"); err = TB_ERR_LIMIT; break; }
       const unsigned cg = (unsigned)(rb * cb);
       if (cplx) crt_kernel<true><<<cg, 32 * kCrtWarps, 0, s>>>(C);

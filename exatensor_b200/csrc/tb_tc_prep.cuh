@@ -52,41 +52,111 @@ int make_operand_map(CUtensorMap* map, const void* base, bool i8, int64_t kpad, 
   return 0;
 }
 
-// ---- offset tables: out[i] = sum_g digit_g(i) * stride_g (first group fastest) --
-struct OffsetParams {
+// ---- offset tables ----------------------------------------------------------------
+// o1[i] = sum_g digit_g(i) s1_g and o2[i] with s2_g, first group fastest.  Rows
+// whose operand is contiguous along another group than D run in blocks of eight
+// of that group (group 0, with its remaining positions the last group): i counts
+// whole blocks first, then the `tail` positions left over, so that no row is
+// padding and both the gathers (eight elements in a row) and the writes of D
+// (rows eight apart) stay coalesced.
+struct TableJob {
   int ng;
-  int64_t count;
-  int64_t ext[kMaxRank];
+  int64_t count, full;        // rows; rows in whole blocks (= count without a tail)
+  int64_t base1, base2;       // offsets of the tail
+  int64_t tail;               // extent of group 0 in the tail
+  FastDiv tail_div;
+  int64_t* o1;
+  int64_t* o2;
+  int64_t ext[kMaxRank], s1[kMaxRank], s2[kMaxRank];
   FastDiv div[kMaxRank];
-  int64_t stride[kMaxRank];
+};
+struct TableParams {
+  TableJob job[3];            // rows of A, rows of B, contracted indices
+  unsigned first[3];          // first CTA of each job
+  unsigned zero_cta;          // first CTA that clears words
+  uint32_t* zero;
+  int64_t zero_words;
 };
 
-__global__ void offsets_kernel(const __grid_constant__ OffsetParams P, int64_t* __restrict__ out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < P.count; i += (int64_t)gridDim.x * blockDim.x) {
-    uint64_t r = (uint64_t)i;
-    int64_t o = 0;
-    for (int g = 0; g < P.ng; ++g) {
-      const uint64_t q = P.div[g].div(r);
-      o += (int64_t)(r - q * (uint64_t)P.ext[g]) * P.stride[g];
+__device__ __forceinline__ void table_job(const TableJob& J, int64_t cta, int64_t ctas) {
+  for (int64_t i = cta * blockDim.x + threadIdx.x; i < J.count; i += ctas * blockDim.x) {
+    const bool tail = i >= J.full;
+    uint64_t r = (uint64_t)(tail ? i - J.full : i);
+    int64_t a = tail ? J.base1 : 0, b = tail ? J.base2 : 0;
+    for (int g = 0; g < J.ng; ++g) {
+      const bool t0 = tail && g == 0;
+      const uint64_t q = t0 ? J.tail_div.div(r) : J.div[g].div(r);
+      const int64_t x = (int64_t)(r - q * (uint64_t)(t0 ? J.tail : J.ext[g]));
+      a += x * J.s1[g];
+      b += x * J.s2[g];
       r = q;
     }
-    out[i] = o;
+    J.o1[i] = a;
+    J.o2[i] = b;
   }
 }
 
-int build_offsets(const std::vector<MGroup>& groups, bool use_s2, int64_t* out, cudaStream_t s) {
-  OffsetParams P;
-  std::memset(&P, 0, sizeof(P));
-  P.ng = (int)groups.size();
-  P.count = 1;
-  for (int g = 0; g < P.ng; ++g) {
-    P.ext[g] = groups[g].ext;
-    P.div[g].init((uint64_t)groups[g].ext);
-    P.stride[g] = use_s2 ? groups[g].s2 : groups[g].s1;
-    P.count *= groups[g].ext;
+// All offset tables of a contraction, and the words that its other kernels
+// expect cleared (row maxima, counters), in one launch.
+__global__ void __launch_bounds__(256) tables_kernel(const __grid_constant__ TableParams P) {
+  const unsigned x = blockIdx.x;
+  if (x >= P.zero_cta) {
+    for (int64_t i = (x - P.zero_cta) * 256 + threadIdx.x; i < P.zero_words; i += (int64_t)(gridDim.x - P.zero_cta) * 256)
+      P.zero[i] = 0;
+  } else if (x >= P.first[2]) {
+    table_job(P.job[2], x - P.first[2], P.zero_cta - P.first[2]);
+  } else if (x >= P.first[1]) {
+    table_job(P.job[1], x - P.first[1], P.first[2] - P.first[1]);
+  } else {
+    table_job(P.job[0], x, P.first[1]);
   }
-  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((P.count + 255) / 256, num_sms() * 8));
-  offsets_kernel<<<(unsigned)blocks, 256, 0, s>>>(P, out);
+}
+
+void set_table_job(TableJob* J, const std::vector<MGroup>& groups, int64_t* o1, int64_t* o2) {
+  J->ng = (int)groups.size();
+  J->count = 1;
+  for (int g = 0; g < J->ng; ++g) {
+    J->ext[g] = groups[g].ext;
+    J->div[g].init((uint64_t)groups[g].ext);
+    J->s1[g] = groups[g].s1;
+    J->s2[g] = groups[g].s2;
+    J->count *= groups[g].ext;
+  }
+  J->full = J->count;
+  J->tail = 1;
+  J->tail_div.init(1);
+  J->o1 = o1;
+  J->o2 = o2;
+}
+
+// Rows in blocks of `block` of group p (see TableJob).
+void set_blocked_job(TableJob* J, const std::vector<MGroup>& groups, int p, int64_t block, int64_t* o1, int64_t* o2) {
+  const MGroup P = groups[p];
+  const int64_t b = std::min(block, P.ext), whole = P.ext / b, rest = P.ext % b;
+  std::vector<MGroup> g;
+  g.push_back({b, P.s1, P.s2, P.dpos, P.src});
+  for (size_t i = 0; i < groups.size(); ++i)
+    if ((int)i != p) g.push_back(groups[i]);
+  g.push_back({whole, P.s1 * b, P.s2 * b, P.dpos, P.src});
+  set_table_job(J, g, o1, o2);
+  if (rest) {
+    J->tail = rest;
+    J->tail_div.init((uint64_t)rest);
+    J->base1 = whole * b * P.s1;
+    J->base2 = whole * b * P.s2;
+    J->count += J->full / b / whole * rest;
+  }
+}
+
+int run_tables(TableParams& P, cudaStream_t s) {
+  unsigned at = 0;
+  for (int j = 0; j < 3; ++j) {
+    P.first[j] = at;
+    at += (unsigned)std::max<int64_t>(1, std::min<int64_t>((P.job[j].count + 255) / 256, num_sms() * 4));
+  }
+  P.zero_cta = at;
+  at += (unsigned)std::max<int64_t>(1, std::min<int64_t>((P.zero_words + 255) / 256, num_sms()));
+  tables_kernel<<<at, 256, 0, s>>>(P);
   TB_CHECK_LAUNCH();
   return 0;
 }
@@ -592,12 +662,28 @@ __device__ __forceinline__ void gather_body(const GatherParams& P, int64_t rowti
   }
 }
 
-// (the complex B' residue mode holds three digit sets per value: two CTAs per
-// SM leave it registers enough not to spill)
-template <int MODE, int NDIG = 3>
-__global__ void __launch_bounds__(kGThreads, MODE == G_RESID_C8B ? 2 : 3)
-    gather_kernel(const __grid_constant__ GatherParams P) {
-  gather_body<MODE, NDIG>(P, blockIdx.x, blockIdx.y, gridDim.y);
+// Both operands of a contraction in one launch: CTAs from ctas_a on work on B.
+// CTA x of an operand takes row tile x % rows and every gy-th K tile from x / rows.
+struct GatherPair {
+  GatherParams a, b;
+  unsigned ctas_a, rows_a, rows_b;
+  int gy_a, gy_b;
+};
+
+// (the complex residue modes leave two CTAs per SM registers enough not to spill)
+template <int MODEA, int MODEB, int NDIG = 3>
+__global__ void __launch_bounds__(kGThreads, MODEB == G_RESID_C8B ? 2 : 3)
+    gather_kernel(const __grid_constant__ GatherPair Q) {
+  const bool second = blockIdx.x >= Q.ctas_a;
+  const unsigned x = second ? blockIdx.x - Q.ctas_a : blockIdx.x, rows = second ? Q.rows_b : Q.rows_a;
+  const unsigned ky = x / rows, rt = x - ky * rows;
+  if constexpr (MODEA == MODEB) {
+    const GatherParams P = second ? Q.b : Q.a;
+    gather_body<MODEA, NDIG>(P, rt, (int)ky, second ? Q.gy_b : Q.gy_a);
+  } else {
+    if (second) gather_body<MODEB, NDIG>(Q.b, rt, (int)ky, Q.gy_b);
+    else gather_body<MODEA, NDIG>(Q.a, rt, (int)ky, Q.gy_a);
+  }
 }
 
 // Grouped form: CTA x works on row tile map[x].y of job map[x].x.
@@ -626,6 +712,22 @@ __global__ void exps_kernel(const unsigned* __restrict__ rowE, int* __restrict__
     const unsigned e = rowE[i / rep];
     out[i] = (int)e - 1021;
     if (list && e >= 2047u && i % rep == 0) list[atomicAdd(count, 1)] = (int)(i / rep);
+  }
+}
+
+// Both operands' exponents in one launch.
+__global__ void exps_pair_kernel(const unsigned* __restrict__ rowE, int* __restrict__ rowx, int64_t m,
+                                 int* __restrict__ badrows, const unsigned* __restrict__ colE, int* __restrict__ colx,
+                                 int64_t n, int rep, int* __restrict__ badcols, int* __restrict__ nbad) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m + n; i += (int64_t)gridDim.x * blockDim.x) {
+    const bool col = i >= m;
+    const int64_t j = col ? i - m : i;
+    const unsigned e = col ? colE[j / rep] : rowE[j];
+    (col ? colx : rowx)[j] = (int)e - 1021;
+    if (e >= 2047u) {
+      if (!col) badrows[atomicAdd(nbad, 1)] = (int)j;
+      else if (j % rep == 0) badcols[atomicAdd(nbad + 1, 1)] = (int)(j / rep);
+    }
   }
 }
 
@@ -741,6 +843,7 @@ struct CrtParams {
   double s1[kMaxModuli], s2[kMaxModuli], s3[kMaxModuli];
   double M1, M2, M3, invM;
   int64_t rows, cols;          // rows of A; columns of B (complex: column pairs)
+  int row_step;                // rows between a warp's lanes (blocked rows: the block, see TableJob)
   const int64_t* dm;
   const int64_t* dn;
   void* D;
@@ -758,9 +861,10 @@ constexpr int kCrtCols = 16, kCrtWarps = 4;
 template <bool CPLX>
 __global__ void __launch_bounds__(32 * kCrtWarps, 3) crt_kernel(const __grid_constant__ CrtParams P) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned row_blocks = (unsigned)((P.rows + 31) / 32);
+  const unsigned rs = (unsigned)P.row_step;
+  const unsigned row_blocks = (unsigned)((P.rows + 32 * rs - 1) / (32 * rs)) * rs;
   const unsigned cb = blockIdx.x / row_blocks, rb = blockIdx.x - cb * row_blocks;
-  const int64_t m = (int64_t)rb * 32 + lane;
+  const int64_t m = ((int64_t)(rb / rs) * 32 + lane) * rs + rb % rs;
   constexpr int RC = CPLX ? 2 : 1, DC = kCrtCols / RC;  // residue columns per D column; D columns per thread
   const int64_t rcols = P.cols * RC;
   const int64_t c0 = ((int64_t)cb * kCrtWarps + warp) * kCrtCols;
@@ -912,8 +1016,12 @@ __device__ __forceinline__ void rowmax_body(const GatherParams& P, int64_t rowti
 }
 
 template <bool CPLX>
-__global__ void __launch_bounds__(kGThreads) rowmax_kernel(const __grid_constant__ GatherParams P) {
-  rowmax_body<CPLX>(P, blockIdx.x, blockIdx.y, gridDim.y);
+__global__ void __launch_bounds__(kGThreads) rowmax_kernel(const __grid_constant__ GatherPair Q) {
+  const bool second = blockIdx.x >= Q.ctas_a;
+  const unsigned x = second ? blockIdx.x - Q.ctas_a : blockIdx.x, rows = second ? Q.rows_b : Q.rows_a;
+  const unsigned ky = x / rows, rt = x - ky * rows;
+  const GatherParams P = second ? Q.b : Q.a;
+  rowmax_body<CPLX>(P, rt, (int)ky, second ? Q.gy_b : Q.gy_a);
 }
 
 template <bool CPLX>
@@ -924,37 +1032,58 @@ __global__ void __launch_bounds__(kGThreads) rowmax_grouped_kernel(const GatherP
   rowmax_body<CPLX>(P, jm.y, blockIdx.y, gridDim.y);
 }
 
+// Grid of a launch over both operands: enough CTAs per operand to fill the GPU
+// several times over, each walking a strided set of K tiles.
+int pair_grid(GatherPair* Q, const GatherParams& a, const GatherParams& b, int64_t rows_a, int64_t kt_a, int64_t rows_b,
+              int64_t kt_b, unsigned* grid) {
+  auto gy = [](int64_t rows, int64_t kt) {
+    return std::max<int64_t>(1, std::min<int64_t>(kt, (int64_t)num_sms() * 16 / std::max<int64_t>(1, rows)));
+  };
+  const int64_t ga = gy(rows_a, kt_a), gb = gy(rows_b, kt_b);
+  if (rows_a * ga + rows_b * gb > INT32_MAX) { set_error("gather grid too large"); return TB_ERR_LIMIT; }
+  Q->a = a;
+  Q->b = b;
+  Q->rows_a = (unsigned)rows_a;
+  Q->rows_b = (unsigned)rows_b;
+  Q->gy_a = (int)ga;
+  Q->gy_b = (int)gb;
+  Q->ctas_a = (unsigned)(rows_a * ga);
+  *grid = (unsigned)(rows_a * ga + rows_b * gb);
+  return 0;
+}
+
 template <bool CPLX>
-int run_rowmax(const GatherParams& P, int64_t grid_rows, int64_t grid_k, cudaStream_t s) {
-  if (grid_rows <= 0 || grid_k <= 0) return 0;
-  if (grid_rows > INT32_MAX) { set_error("gather grid too large"); return TB_ERR_LIMIT; }
-  int64_t gy = std::max<int64_t>(1, std::min<int64_t>(grid_k, (int64_t)num_sms() * 16 / std::max<int64_t>(1, grid_rows)));
-  gy = std::min<int64_t>(gy, 65535);
-  rowmax_kernel<CPLX><<<dim3((unsigned)grid_rows, (unsigned)gy), kGThreads, 0, s>>>(P);
+int run_rowmax(const GatherParams& a, const GatherParams& b, cudaStream_t s) {
+  constexpr int64_t TM = CPLX ? gather_rows<double2>() : gather_rows<double>();
+  GatherPair Q;
+  unsigned grid;
+  if (int e = pair_grid(&Q, a, b, (a.rows + TM - 1) / TM, (a.K + kGK - 1) / kGK, (b.rows + TM - 1) / TM,
+                        (b.K + kGK - 1) / kGK, &grid))
+    return e;
+  rowmax_kernel<CPLX><<<grid, kGThreads, 0, s>>>(Q);
   TB_CHECK_LAUNCH();
   return 0;
 }
 
-template <int MODE>
-int run_gather(const GatherParams& P, int64_t grid_rows, int64_t grid_k, cudaStream_t s) {
-  if (grid_rows <= 0 || grid_k <= 0) return 0;
-  if (grid_rows > INT32_MAX) { set_error("gather grid too large"); return TB_ERR_LIMIT; }
-  // enough CTAs to fill the GPU several times over; each walks a strided set of K tiles
-  int64_t gy = std::max<int64_t>(1, std::min<int64_t>(grid_k, (int64_t)num_sms() * 16 / std::max<int64_t>(1, grid_rows)));
-  gy = std::min<int64_t>(gy, 65535);
-  constexpr int smem = gather_smem_bytes<MODE>();
+template <int MODEA, int MODEB>
+int run_gather(const GatherParams& a, const GatherParams& b, int64_t rows_a, int64_t rows_b, int64_t ktiles,
+               cudaStream_t s) {
+  GatherPair Q;
+  unsigned grid;
+  if (int e = pair_grid(&Q, a, b, rows_a, ktiles, rows_b, ktiles, &grid)) return e;
+  constexpr int smem = std::max(gather_smem_bytes<MODEA>(), gather_smem_bytes<MODEB>());
   auto launch = [&](auto kern, DeviceOnce& once) -> int {
     const cudaError_t e = smem_limit_once(once, kern, smem);
     if (e != cudaSuccess) { set_error("gather smem attribute: %s", cudaGetErrorString(e)); return TB_ERR_CUDA; }
-    kern<<<dim3((unsigned)grid_rows, (unsigned)gy), kGThreads, smem, s>>>(P);
+    kern<<<grid, kGThreads, smem, s>>>(Q);
     return 0;
   };
   static DeviceOnce once3, once4;
   int err = 0;
-  if constexpr (MODE == G_RESID_R8 || MODE == G_RESID_C8A || MODE == G_RESID_C8B) {
-    err = P.rs.ndig > 3 ? launch(gather_kernel<MODE, 4>, once4) : launch(gather_kernel<MODE, 3>, once3);
+  if constexpr (MODEA == G_RESID_R8 || MODEA == G_RESID_C8A) {
+    err = a.rs.ndig > 3 ? launch(gather_kernel<MODEA, MODEB, 4>, once4) : launch(gather_kernel<MODEA, MODEB, 3>, once3);
   } else {
-    err = launch(gather_kernel<MODE>, once3);
+    err = launch(gather_kernel<MODEA, MODEB>, once3);
   }
   if (err) return err;
   TB_CHECK_LAUNCH();
