@@ -10,7 +10,8 @@
 //    permutations with the conversion to tensor-core formats and the epilogue
 //    writes D through the output permutation with alpha/beta applied.
 //  * the one-kernel form (tb_direct.cu): the plain method's arithmetic without
-//    its permutation passes, for what TB_METHOD_AUTO would run as TTGT.
+//    its permutation passes, for what TB_METHOD_AUTO would run as TTGT (long R8
+//    and C8 products go to the tensor cores with 15 moduli instead).
 // A full contraction into a scalar (D rank 0) uses a deterministic two-pass
 // dot-product kernel (the reference's gpu_array_dot_product__, :531).
 #include "tb_common.cuh"
@@ -350,24 +351,46 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
     unsigned tune = 0;
     uint64_t key = 0;
     descriptor_of(Z, dtk, f);
-    // The plain method in one kernel, in the tensors' own layouts: the same FP64
-    // or wider sums without the permutation passes and their scratch.  On random
-    // contractions of the four kinds it ran 1.1 to 7 times as fast as TTGT (8 to
-    // 30 us instead of 27 to 100 us for small ones).  TTGT keeps the products
-    // that the FP64 tensor rate bounds, where its larger tiles read the operands
-    // less often (1980 x 1881 x 816: 327 us against 342 us).  Where the tensor
-    // cores are picked, one kernel still replaces them when it is predicted to
-    // take less than their launches alone: about 16 kernels, 60 us or more for
-    // the smallest product (K = 9856, M = N = 150: 147 us against 67 us), unless
-    // the plan asks for details of that path.
-    auto try_direct = [&](int picked, int* err) {
-      constexpr double kFusedLaunchesUs = 50.0;
+    // What the library makes of a picked method, for a plan that asks for no
+    // details:
+    //  * The plain method runs in one kernel in the tensors' own layouts
+    //    (tb_direct.cu): the same FP64 or wider sums without permutation passes
+    //    and scratch, 1.1 to 7 times as fast as TTGT over random contractions (8
+    //    to 30 us instead of 27 to 100 us for small ones).
+    //  * R8 and C8 products picked plain but long enough run as residues with 15
+    //    moduli, 51 or 52 operand bits, where that is predicted faster: 96/24
+    //    ladder 4.04 -> 1.59 ms, 1600^3 475 -> 210 us.  Their error is below the
+    //    plain sums' from K = 256 on (relative to long double, uniform data: 5e-17
+    //    against 5e-16 at K = 256, 1.3e-15 at 1600; normal data 4e-16 against 5e-16
+    //    and 1.4e-15), because nothing rounds inside a sum.
+    //  * A product picked for the tensor cores runs in one kernel where that is
+    //    predicted faster than their preparation alone (K = 9856, M = N = 150: 147
+    //    us against 67 us).
+    // A network of the caller's own keeps its choice of the tensor cores.  The
+    // predictions are fits to measured times (about 5% and 15% off).
+    auto refine = [&](int picked, bool callers, int* err) {
       const bool asked = plan && (plan->slices || plan->tile_n || plan->tile_m || plan->bf16_terms || plan->moduli);
-      if (picked == TB_METHOD_FUSED && asked) return false;
-      if (picked == TB_METHOD_TTGT && dtk == kR8 && Z.M >= 1792 && Z.N >= 1792 && Z.K >= 512) return false;
+      if (picked == TB_METHOD_FUSED && (asked || callers)) return false;
       DirectPlan dp;
-      if (direct_plan(Z, dtk, d, l, r, &dp) != 0) return false;
-      if (picked == TB_METHOD_FUSED && dp.us >= kFusedLaunchesUs) return false;
+      const bool direct_ok = direct_plan(Z, dtk, d, l, r, &dp) == 0;
+      const int64_t Kr = cplx ? 2 * Z.K : Z.K;
+      constexpr int64_t kExactMinK = 256;
+      if (picked == TB_METHOD_TTGT && is_double(dtk) && !callers && !asked && Kr >= kExactMinK &&
+          predicted_fused_us(Z, dtk, 15) < (direct_ok ? dp.us : 1e30)) {
+        tb_plan_t rp{};
+        rp.method = TB_METHOD_FUSED;
+        rp.moduli = 15;
+        const int fe = contract_fused(Z, dtk, ddims, d, ldims, l, rdims, r, ar, ai, accumulative != 0, lconj, rconj, &rp,
+                                      s, &g_stats);
+        // short of scratch, or K beyond the pass table: as before
+        if (fe != TB_ERR_NO_MEMORY && fe != TB_ERR_NOT_IMPLEMENTED && fe != TB_ERR_LIMIT && fe != TB_ERR_INVALID_ARGS) {
+          g_stats.method = TB_METHOD_FUSED;
+          *err = fe;
+          return true;
+        }
+      }
+      if (!direct_ok) return false;
+      if (picked == TB_METHOD_FUSED && dp.us >= predicted_fused_us(Z, dtk, 14)) return false;
       g_stats.method = TB_METHOD_TTGT;
       g_stats.gemm_launches = 1;
       *err = run_direct(dp, dtk, cplx ? ar : real_alpha(ar, ai), cplx ? ai : 0.0, accumulative != 0, lconj, rconj, s);
@@ -440,14 +463,13 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
         g_stats.m = Z.M; g_stats.n = Z.N; g_stats.k = Z.K;
         g_stats.flops = (cplx ? 8.0 : 2.0) * (double)Z.M * (double)Z.N * (double)Z.K;
       }
-      const bool mine = !selector_is_callers();
-      if ((idx == 0 || mine) && try_direct(idx == 0 ? TB_METHOD_TTGT : TB_METHOD_FUSED, &e)) return e;
+      if (refine(idx == 0 ? TB_METHOD_TTGT : TB_METHOD_FUSED, selector_is_callers(), &e)) return e;
       learned = candidate(idx);
       return run_method(Z, dtk, ddims, d, ldims, l, rdims, r, ar, ai, accumulative, lconj, rconj, &learned, s,
                         /*fallback=*/true);
     }
     method = select_method(dtk, Z, plan);
-    if (try_direct(method, &e)) return e;
+    if (refine(method, false, &e)) return e;
   }
   if (method == TB_METHOD_AUTO) method = TB_METHOD_TTGT;
   learned = plan ? *plan : tb_plan_t{};

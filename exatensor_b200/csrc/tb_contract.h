@@ -20,6 +20,9 @@ int contract_fused(const Matricization& Z, int dtk, const int* ddims, void* d, c
                    const int* rdims, const void* r, double ar, double ai, bool accumulate, int lconj, int rconj,
                    const tb_plan_t* plan, cudaStream_t s, tb_contract_stats_t* stats);
 
+// Predicted microseconds of contract_fused's default plan (R8, C8: n moduli).
+double predicted_fused_us(const Matricization& Z, int dtk, int n);
+
 // Learned plan selection (tb_select.cu).
 int descriptor_of(const Matricization& Z, int dtk, float* features);
 // -1 when no selector is installed; else 0 with the chosen plan index, whether

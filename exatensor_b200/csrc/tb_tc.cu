@@ -226,6 +226,39 @@ int select_method(int dtk, const Matricization& Z, const tb_plan_t* plan) {
   return TB_METHOD_TTGT;
 }
 
+// Fixed launches, operand bytes read and plane bytes written (MB), MMA work of
+// whole rounds of work units (10^6 operations), output bytes (MB) and rounds,
+// weighted by a fit to 212 random contractions on B200 (5% rms for R8, 8% for
+// R4): a round of units costs its MMAs plus about 3 us, D's bytes run at 2.6 to
+// 4.4 TB/s, operands at 4 to 7 TB/s.
+double predicted_fused_us(const Matricization& Z, int dtk, int n) {
+  const bool cplx = is_complex(dtk), f64 = is_double(dtk);
+  bool swap = false;  // rows: the operand holding D's fastest dimension
+  {
+    int64_t lm = INT64_MAX, ln = INT64_MAX;
+    for (auto& g : Z.m) if (g.ext > 1) lm = std::min(lm, g.s2);
+    for (auto& g : Z.n) if (g.ext > 1) ln = std::min(ln, g.s2);
+    swap = ln < lm;
+  }
+  const double M = (double)(swap ? Z.N : Z.M), N = (double)(swap ? Z.M : Z.N), K = (double)Z.K, es = elem_bytes(dtk);
+  const double Kr = cplx ? 2 * K : K, Nr = cplx ? 2 * N : N;
+  const double bn = Nr >= 192 ? 256 : 128;
+  const double mt = std::ceil(M / 128), nt = std::ceil(Nr / bn), kp = std::ceil(Kr / 128) * 128;
+  const double reads = f64 ? 2 : 1, plane = f64 ? n : 4;  // row maxima read FP64 operands a second time
+  const double gather = ((M + N) * K * es * reads + (mt * 128 + nt * bn) * kp * plane) * 1e-6;
+  const double sms = 148;
+  if (f64) {
+    const double rounds = std::ceil(n * mt * nt / sms);
+    const double work = rounds * sms * 128 * bn * kp * 2e-6, out = M * Nr * (n + 16) * 1e-6;
+    return cplx ? 41.3 + 0.23 * gather + 0.000275 * work + 0.271 * out + 3.53 * rounds
+                : 44.4 + 0.271 * gather + 0.000293 * work + 0.384 * out + 3.33 * rounds;
+  }
+  const double passes = std::ceil(std::ceil(Kr * 2 / 128) / 32), rounds = std::ceil(mt * nt / sms);
+  const double work = rounds * sms * 128 * bn * kp * 6e-6, out = M * Nr * 8 * passes * 1e-6;
+  return cplx ? 27.0 + 0.135 * gather + 0.000448 * work + 0.144 * out + 9.19 * rounds * passes
+              : 30.5 + 0.224 * gather + 0.000437 * work + 0.331 * out + 14.8 * rounds * passes;
+}
+
 int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, const int* ldims, const void* l,
                    const int* rdims, const void* r, double ar, double ai, bool accumulate, int lconj, int rconj,
                    const tb_plan_t* plan, cudaStream_t s, tb_contract_stats_t* stats) {
