@@ -381,6 +381,39 @@ int build_perm_plan_o2n(int es, int rank, const int* dims, const int* cptrn, Per
   return build_perm_plan(es, rank, D, SI, SO, p, vmin_kb, vmax_kb, min_run);
 }
 
+bool build_elem_plan(int es, int rank, const int* dims, const int* cptrn, int64_t max_bytes, ElemPermParams* P) {
+  if (rank < 0 || rank > kPlanMaxRank) return false;
+  int64_t vol = 1, sin[kPlanMaxRank];
+  int at[kPlanMaxRank];
+  for (int i = 0; i < rank; ++i) at[i] = -1;
+  for (int i = 0; i < rank; ++i) {
+    if (dims[i] < 1 || cptrn[i] < 1 || cptrn[i] > rank || at[cptrn[i] - 1] >= 0) return false;
+    at[cptrn[i] - 1] = i;
+    sin[i] = vol;
+    vol *= dims[i];
+    if (vol * es > max_bytes || vol >= ((int64_t)1 << 31) - (1 << 20)) return false;
+  }
+  // output order, unit extents dropped, neighbours in both orders merged
+  int r = 0;
+  for (int q = 0; q < rank; ++q) {
+    const int i = at[q];
+    if (dims[i] == 1) continue;
+    if (r && (int64_t)P->sin[r - 1] * P->ext[r - 1] == sin[i]) {
+      P->ext[r - 1] *= (uint32_t)dims[i];
+      continue;
+    }
+    if (r == kElemRank) return false;
+    P->ext[r] = (uint32_t)dims[i];
+    P->sin[r] = (uint32_t)sin[i];
+    ++r;
+  }
+  if (!r) { P->ext[0] = P->sin[0] = 1; r = 1; }
+  P->rank = r;
+  P->vol = (uint32_t)vol;
+  for (int d = 0; d < r; ++d) magic32(P->ext[d], &P->magic[d], &P->shift[d]);
+  return true;
+}
+
 int perm_glist_vector_bytes(const PermParams& P, int in_align, int nthr) {
   const int es = P.es;
   int vb = es;

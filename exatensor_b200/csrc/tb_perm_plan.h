@@ -119,6 +119,28 @@ int perm2d_list_entries(const PermParams& P, bool rows, int nthr);
 // load copies per tile, or tile-relative offsets beyond 32 bits).
 constexpr int kGListEntries = 16;
 int perm_glist_vector_bytes(const PermParams& P, int in_align, int nthr);
+// Element permutations (elem_perm_kernel): the dims in output order, first fastest,
+// with their input strides; output element i is the input element at sum of digit_d
+// (i) * sin[d], the last dim's digit being what is left of i.
+constexpr int kElemRank = 16;
+struct ElemPermParams {
+  int rank;
+  uint32_t vol;
+  uint32_t ext[kElemRank], magic[kElemRank];
+  int shift[kElemRank];
+  uint32_t sin[kElemRank];
+};
+// Takes dim d's digit off *rest and adds its input offset.
+TB_HD void elem_digit(const ElemPermParams& P, int d, uint32_t* rest, uint32_t* off) {
+  const uint32_t q = fdiv32(*rest, P.magic[d], P.shift[d]);
+  *off += (*rest - q * P.ext[d]) * P.sin[d];
+  *rest = q;
+}
+// Plans the element kernel for an O2N permutation of a tensor of at most max_bytes
+// (and 2^31 - 2^20 elements, kElemRank dims after merging).  False otherwise, and
+// for a pattern that is no permutation (the general path reports it).
+bool build_elem_plan(int es, int rank, const int* dims, const int* cptrn, int64_t max_bytes, ElemPermParams* P);
+
 // Bytes of one pipeline stage (a tile in shared memory).
 inline int64_t perm_stage_bytes(const PermParams& P) { return (int64_t)P.nA * P.lap * P.es; }
 

@@ -36,6 +36,51 @@ __global__ void scatter_kernel(const __grid_constant__ ScatterParams P, const E*
   }
 }
 
+// ---------------------------------------------------------------------------
+// Element permutations: a thread computes the input offset of each output element
+// that it writes and moves it, without tiles, tables or shared memory; threads run
+// along the output.  A call costs little more than its launch (the tiled engine's
+// 11 KB of parameters and per-thread offset lists take 3 us, which bounds it on
+// tensors of a few megabytes), and independent threads keep more bytes in flight
+// than the tiled engine's stages, which bounds its additions.  What bounds this
+// kernel is one sector read from L2 per element that is not contiguous in the
+// input, and about ten instructions per dimension: R8 random permutations of 16 MB,
+// copy 15.8 -> 10.9 us and addition 25.8 -> 12.5 us.  Reading the input in 64-byte
+// blocks instead (a second output offset per element) cost more instructions than
+// its sectors saved: 18.6 us.
+// ---------------------------------------------------------------------------
+constexpr int kElemUnroll = 4;
+
+template <typename E, typename Store>
+__global__ void __launch_bounds__(256) elem_perm_kernel(const __grid_constant__ ElemPermParams P,
+                                                        const E* __restrict__ in, Store st) {
+  const uint32_t first = blockIdx.x * (256u * kElemUnroll) + threadIdx.x;
+  uint32_t off[kElemUnroll], rest[kElemUnroll];
+#pragma unroll
+  for (int u = 0; u < kElemUnroll; ++u) { off[u] = 0; rest[u] = first + u * 256u; }
+  for (int d = 0; d < P.rank - 1; ++d) {
+#pragma unroll
+    for (int u = 0; u < kElemUnroll; ++u) elem_digit(P, d, &rest[u], &off[u]);
+  }
+  const uint32_t last = P.sin[P.rank - 1];
+  E v[kElemUnroll];
+  typename rmw_old<Store, E>::type old[kElemUnroll];
+#pragma unroll
+  for (int u = 0; u < kElemUnroll; ++u) {
+    const uint32_t o = first + u * 256u;
+    if (o >= P.vol) continue;
+    v[u] = in[off[u] + rest[u] * last];
+    if constexpr (is_rmw_store<Store>::value) old[u] = st.load(o);
+  }
+#pragma unroll
+  for (int u = 0; u < kElemUnroll; ++u) {
+    const uint32_t o = first + u * 256u;
+    if (o >= P.vol) continue;
+    if constexpr (is_rmw_store<Store>::value) st.put(o, v[u], old[u]);
+    else st(o, v[u]);
+  }
+}
+
 namespace {
 
 int o2n_strides(int rank, const int* dims, const int* cptrn, int64_t* sout) {
@@ -74,6 +119,33 @@ int run_scatter(int rank, const int* dims, const int* cptrn, const E* in, const 
   int64_t blocks = std::min<int64_t>((vol + 255) / 256, (int64_t)num_sms() * 16);
   if (blocks < 1) blocks = 1;
   scatter_kernel<E, Store><<<(unsigned)blocks, 256, 0, s>>>(P, in, st);
+  TB_CHECK_LAUNCH();
+  return 0;
+}
+
+// Bytes of a tensor up to which the element kernel runs: where, over random
+// permutations of ranks 2 to 6 with inputs that change from call to call, it stops
+// being ahead of the tiled engine.  Mean us, tiled against element: copies of
+// 4-byte elements 29.0 / 26.5 at 24 MB and 25.9 / 28.3 at 32 MB, of 8-byte ones 23.0
+// / 19.1 at 32 MB, of 16-byte ones 17.5 / 15.5 at 32 MB; additions 84.6 / 66.2 at 64
+// MB and 206 / 232 at 128 MB, 88 / 81 at 128 MB and 183 / 211 at 260 MB, 175 / 121 at
+// 260 MB.  Copies of 32 MB or more time it beside the other plans; additions
+// are never timed.
+constexpr int64_t elem_limit(int es, bool rmw) {
+  return rmw ? (es == 4 ? (int64_t)64 << 20 : es == 8 ? (int64_t)128 << 20 : (int64_t)272 << 20)
+             : (es == 4 ? (int64_t)24 << 20 : ((int64_t)32 << 20) - 1);
+}
+
+// TB_PERM_LOADS (a tuning knob) names a load mechanism of the tiled engine: no
+// element kernel then.
+bool elem_allowed() {
+  static const bool on = !getenv("TB_PERM_LOADS");
+  return on;
+}
+
+template <typename E, typename Store>
+int launch_elem(const ElemPermParams& P, const E* in, const Store& st, cudaStream_t s) {
+  elem_perm_kernel<E, Store><<<(P.vol + 256 * kElemUnroll - 1) / (256 * kElemUnroll), 256, 0, s>>>(P, in, st);
   TB_CHECK_LAUNCH();
   return 0;
 }
@@ -168,7 +240,10 @@ constexpr int kBulkRowsCand = kNumTileCandidates;
 // the TMA-staged transpose kernel (tb_perm_tma.cuh) on the default plan's
 // reduced view, where its layout requirements hold
 constexpr int kTmaCand = kNumTileCandidates + 1;
-constexpr int kNumPlanCandidates = kNumTileCandidates + 2;
+// the element kernel
+constexpr int kElemCand = kNumTileCandidates + 2;
+constexpr int64_t kElemCandBytes = (int64_t)128 << 20;  // far behind on larger copies: not worth timing
+constexpr int kNumPlanCandidates = kNumTileCandidates + 3;
 
 bool long_row_copy(const PermParams& P) { return P.rows2d && P.tma_ok && (int64_t)P.LA * P.es >= 4096; }
 
@@ -192,6 +267,14 @@ bool same_work(const PermParams& a, const PermParams& b) {
 
 template <typename E, typename Store>
 int run_copy_measured(int rank, const int* dims, const int* cptrn, const E* in, const Store& st, cudaStream_t s) {
+  // TB_PERM_TMA=1 / 0: the TMA-staged kernel wherever it applies / never
+  // (tuning and test switch; results are identical)
+  static const int tma_env = [] { const char* e = getenv("TB_PERM_TMA"); return e ? (e[0] == '1' ? 1 : 0) : -1; }();
+  ElemPermParams S;
+  if (tma_env != 1 && elem_allowed()) {
+    if (build_elem_plan((int)sizeof(E), rank, dims, cptrn, elem_limit(sizeof(E), is_rmw_store<Store>::value), &S))
+      return launch_elem<E, Store>(S, in, st, s);
+  }
   int64_t vol = 1;
   for (int i = 0; i < rank; ++i) vol *= dims[i];
   std::vector<int> key{(int)sizeof(E), rank};
@@ -206,14 +289,13 @@ int run_copy_measured(int rank, const int* dims, const int* cptrn, const E* in, 
   static const bool tune_on = [] { const char* e = getenv("TB_PERM_TUNE"); return !(e && e[0] == '0'); }();
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) { cudaGetLastError(); cap = cudaStreamCaptureStatusActive; }
-  // TB_PERM_TMA=1 / 0: the TMA-staged kernel wherever it applies / never
-  // (tuning and test switch; results are identical)
-  static const int tma_env = [] { const char* e = getenv("TB_PERM_TMA"); return e ? (e[0] == '1' ? 1 : 0) : -1; }();
   const bool tune = pick < 0 && tune_on && tma_env < 0 && vol * (int64_t)sizeof(E) >= kTuneMinBytes &&
                     cap == cudaStreamCaptureStatusNone;
   if (!tune) {
     const int c = tma_env == 1 ? kTmaCand : (pick < 0 ? 0 : pick);
-    const TileBounds b = kTileCandidates[(c == kBulkRowsCand || c == kTmaCand) ? 0 : c];
+    if (c == kElemCand && build_elem_plan((int)sizeof(E), rank, dims, cptrn, kElemCandBytes, &S))
+      return launch_elem<E, Store>(S, in, st, s);
+    const TileBounds b = kTileCandidates[c >= kNumTileCandidates ? 0 : c];
     PermParams P;
     int e = build_perm_plan_o2n((int)sizeof(E), rank, dims, cptrn, &P, b.vmin_kb, b.vmax_kb, b.min_run);
     if (e == 0) {
@@ -249,14 +331,17 @@ int run_copy_measured(int rank, const int* dims, const int* cptrn, const E* in, 
   }
   static TmaPermParams tma;  // large (a tensor map); built under the lock
   const bool with_tma = tma_perm_plan(plans[0], in, &tma);
-  if (n == 1 && !with_tma) { remember_choice(key, 0); return launch_perm<E, Store>(plans[0], in, st, s); }
+  const bool with_elem = elem_allowed() && build_elem_plan((int)sizeof(E), rank, dims, cptrn, kElemCandBytes, &S);
+  if (n == 1 && !with_tma && !with_elem) { remember_choice(key, 0); return launch_perm<E, Store>(plans[0], in, st, s); }
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess) { set_error("cudaEventCreate failed"); return TB_ERR_CUDA; }
   if (cudaEventCreate(&e1) != cudaSuccess) { cudaEventDestroy(e0); set_error("cudaEventCreate failed"); return TB_ERR_CUDA; }
   float best_ms = 0.f, ms0 = 0.f;
   int best = 0, err = 0;
   if (with_tma) idx[n++] = kTmaCand;
+  if (with_elem) idx[n++] = kElemCand;
   auto run = [&](int k) {
+    if (idx[k] == kElemCand) return launch_elem<E, Store>(S, in, st, s);
     return idx[k] == kTmaCand ? launch_perm_tma<E, Store>(tma, st, s) : launch_perm<E, Store>(plans[k], in, st, s);
   };
   for (int k = 0; k < n && !err; ++k) {
@@ -296,6 +381,10 @@ template <typename E, typename Store>
 int run_permutation(int rank, const int* dims, const int* cptrn, const E* in, const Store& st,
                     cudaStream_t s, bool force_scatter = false) {
   if (!force_scatter) {
+    ElemPermParams S;
+    if (elem_allowed() &&
+        build_elem_plan((int)sizeof(E), rank, dims, cptrn, elem_limit(sizeof(E), is_rmw_store<Store>::value), &S))
+      return launch_elem<E, Store>(S, in, st, s);
     std::vector<int> key{(int)sizeof(E), rank};
     key.insert(key.end(), dims, dims + rank);
     key.insert(key.end(), cptrn, cptrn + rank);
@@ -305,7 +394,7 @@ int run_permutation(int rank, const int* dims, const int* cptrn, const E* in, co
       auto it = g_tune.find(key);
       if (it != g_tune.end()) pick = it->second;
     }
-    const TileBounds b = kTileCandidates[(pick < 0 || pick == kBulkRowsCand || pick == kTmaCand) ? 0 : pick];
+    const TileBounds b = kTileCandidates[(pick < 0 || pick >= kNumTileCandidates) ? 0 : pick];
     PermParams P;
     int e = build_perm_plan_o2n((int)sizeof(E), rank, dims, cptrn, &P, b.vmin_kb, b.vmax_kb, b.min_run);
     for (int c : {kListCand, kListCandShort}) {
