@@ -51,10 +51,14 @@ struct OpBlock {          // one distinct operand block in the A (row) or B (col
   size_t plane_off;               // bytes into the plane buffer
 };
 
-void* dalloc(size_t bytes, int* err) {
+// Plan memory from the device's pool, which keeps what earlier plans gave back
+// (cudaMalloc maps fresh memory each time: 2 ms for a few hundred MB).  Plans are
+// created on one stream and used on others: creation ends with a synchronization,
+// and a plan's memory goes back only after the device is idle.
+void* dalloc(size_t bytes, int* err, cudaStream_t s) {
   void* p = nullptr;
   if (*err) return nullptr;
-  if (cudaMalloc(&p, std::max<size_t>(bytes, 256)) != cudaSuccess) {
+  if (cudaMallocAsync(&p, std::max<size_t>(bytes, 256), s) != cudaSuccess) {
     cudaGetLastError();
     set_error("block-sparse plan: device allocation of %zu bytes failed", bytes);
     *err = TB_ERR_NO_MEMORY;
@@ -69,6 +73,11 @@ void* dalloc(size_t bytes, int* err) {
 struct tb_bsc_plan_s {
   int dtk = 0;
   bool i8 = true;
+  bool resid = false;              // FP64 by modular residues (else INT8 slices)
+  tb::ResiduePlan rp;              // residues: moduli and reconstruction constants
+  tb::CrtView* crt_views = nullptr;  // residues: one per output block
+  int2* crt_map = nullptr;         // residues: CTA -> (output block, block of it)
+  int64_t crt_ctas = 0;
   int slices = 6, bn = 256;        // current configuration
   int max_slices = 7;              // planes allocated for this many slices
   double ar = 1, ai = 0, br = 0, bi = 0;
@@ -140,9 +149,14 @@ int bsc_enqueue(tb_bsc_plan_s* pl, cudaStream_t s) {
     TB_CHECK_LAUNCH();
   }
   // the gathers read the slice count from the jobs: keep them in sync with the configuration
-  const cudaError_t ga = pl->i8 ? gather_grouped_prepare<G_SLICE_R8>() : gather_grouped_prepare<G_SPLIT_R4>();
+  const cudaError_t ga = pl->resid ? gather_grouped_prepare<G_RESID_R8>()
+                         : pl->i8  ? gather_grouped_prepare<G_SLICE_R8>()
+                                   : gather_grouped_prepare<G_SPLIT_R4>();
   if (ga != cudaSuccess) { set_error("grouped gather smem attribute: %s", cudaGetErrorString(ga)); return TB_ERR_CUDA; }
-  if (pl->i8)
+  if (pl->resid)
+    gather_grouped_kernel<G_RESID_R8><<<dim3((unsigned)pl->g_ctas, (unsigned)pl->g_gy), kGThreads,
+                                        gather_smem_bytes<G_RESID_R8>(), s>>>(pl->jobs, pl->g_map);
+  else if (pl->i8)
     gather_grouped_kernel<G_SLICE_R8><<<dim3((unsigned)pl->g_ctas, (unsigned)pl->g_gy), kGThreads,
                                         gather_smem_bytes<G_SLICE_R8>(), s>>>(pl->jobs, pl->g_map);
   else
@@ -157,11 +171,19 @@ int bsc_enqueue(tb_bsc_plan_s* pl, cudaStream_t s) {
   P.passes = pl->passes; P.runs = pl->runs;
   P.ar = pl->ar; P.ai = pl->ai; P.br = pl->br; P.bi = pl->bi;
   P.err = device_error_word();
-  const int grid = std::max(1, std::min(P.nitems, num_sms()));
-  int e;
-  if (pl->bn == 256) e = pl->i8 ? launch_bsc<256, true, EPI_OZAKI_R>(P, grid, s) : launch_bsc<256, false, EPI_BF16_R>(P, grid, s);
-  else e = pl->i8 ? launch_bsc<128, true, EPI_OZAKI_R>(P, grid, s) : launch_bsc<128, false, EPI_BF16_R>(P, grid, s);
-  return e;
+  P.moduli = pl->resid ? pl->rp.rs.n : 1;
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)P.nitems * P.moduli, num_sms()));
+  if (pl->resid) {
+    if (int e = pl->bn == 256 ? launch_bsc<256, true, EPI_RESID>(P, grid, s) : launch_bsc<128, true, EPI_RESID>(P, grid, s))
+      return e;
+    CrtParams C = pl->rp.crt;
+    C.ar = pl->ar; C.ai = pl->ai; C.br = pl->br; C.bi = pl->bi;
+    crt_grouped_kernel<<<(unsigned)pl->crt_ctas, 32 * kCrtWarps, 0, s>>>(C, pl->crt_views, pl->crt_map);
+    TB_CHECK_LAUNCH();
+    return 0;
+  }
+  if (pl->bn == 256) return pl->i8 ? launch_bsc<256, true, EPI_OZAKI_R>(P, grid, s) : launch_bsc<256, false, EPI_BF16_R>(P, grid, s);
+  return pl->i8 ? launch_bsc<128, true, EPI_OZAKI_R>(P, grid, s) : launch_bsc<128, false, EPI_BF16_R>(P, grid, s);
 }
 
 void drop_graph(tb_bsc_plan_s* pl) {
@@ -187,7 +209,9 @@ void plan_passes(const tb_bsc_plan_s* pl, int S, std::vector<BscPass>& passes, s
   passes.clear();
   runs.clear();
   const bool maps = !pl->pair_maps.empty();
-  auto new_pass = [&](int shift) { passes.push_back(BscPass{(int)runs.size(), 0, shift, 0}); };
+  auto new_pass = [&](int shift) {
+    passes.push_back(BscPass{(int)runs.size(), 0, shift, shift > 1 ? (int)(4294967296ull / (unsigned)shift) : 0});
+  };
   // run of global pair q over K blocks [k0, k1) in planes (a, b), added to the last pass
   auto add_run = [&](int q, int a, int b, int k0, int k1) {
     BscRun r{};
@@ -204,7 +228,12 @@ void plan_passes(const tb_bsc_plan_s* pl, int S, std::vector<BscPass>& passes, s
     const std::vector<int>& kb = pl->dpair_kb[d];
     const int p0 = pl->dpair0[d], np = (int)kb.size();
     const int pass0 = (int)passes.size(), run0 = (int)runs.size();
-    if (!pl->i8) {
+    if (pl->resid) {
+      for (int i = 0; i < pl->rp.rs.n; ++i) {
+        new_pass(pl->rp.crt.mod[i]);
+        for (int q = 0; q < np; ++q) add_run(p0 + q, i, i, 0, kb[q]);
+      }
+    } else if (!pl->i8) {
       int load = kBscBf16PassKBlocks;  // forces a new pass first
       for (int q = 0; q < np; ++q) {
         for (int k0 = 0; k0 < kb[q];) {
@@ -292,13 +321,14 @@ namespace {
 
 void plan_free(tb_bsc_plan_s* pl) {
   drop_graph(pl);
-  for (void* p : pl->allocs) cudaFree(p);
+  if (!pl->allocs.empty()) cudaDeviceSynchronize();
+  for (void* p : pl->allocs) cudaFreeAsync(p, 0);
   delete pl;
 }
 
 template <typename T>
 T* upload(tb_bsc_plan_s* pl, const std::vector<T>& v, int* err, cudaStream_t s) {
-  T* d = (T*)dalloc(sizeof(T) * std::max<size_t>(1, v.size()), err);
+  T* d = (T*)dalloc(sizeof(T) * std::max<size_t>(1, v.size()), err, s);
   if (!d) return nullptr;
   pl->allocs.push_back(d);
   if (!v.empty() && cudaMemcpyAsync(d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, s) != cudaSuccess) {
@@ -309,8 +339,13 @@ T* upload(tb_bsc_plan_s* pl, const std::vector<T>& v, int* err, cudaStream_t s) 
   return d;
 }
 
+// Residue planes of a plan (operands and output): 14 bytes per operand element
+// against 6 of the slices, and 14 per output element.  Plans that would need more
+// than this keep the slices.
+constexpr size_t kBscResidueBytes = (size_t)24 << 30;
+
 int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t* tasks, double ar, double ai,
-                int accumulative, const tb_plan_t* plan, tb_bsc_plan_s** out, cudaStream_t s) {
+                int accumulative, const tb_plan_t* plan, tb_bsc_plan_s** out, cudaStream_t s, bool allow_residues) {
   *out = nullptr;
   if (!pattern || !tasks || ntasks < 1) { set_error("tb_bsc_plan_create: no tasks"); return TB_ERR_INVALID_ARGS; }
   if (dtk != kR8 && dtk != kR4) {
@@ -333,7 +368,8 @@ int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t*
   pl->i8 = dtk == kR8;
   {
     // attribute set here, before any graph capture of the plan's launches
-    const cudaError_t ga = pl->i8 ? gather_grouped_prepare<G_SLICE_R8>() : gather_grouped_prepare<G_SPLIT_R4>();
+    cudaError_t ga = pl->i8 ? gather_grouped_prepare<G_SLICE_R8>() : gather_grouped_prepare<G_SPLIT_R4>();
+    if (ga == cudaSuccess && pl->i8) ga = gather_grouped_prepare<G_RESID_R8>();
     if (ga != cudaSuccess) {
       set_error("grouped gather smem attribute: %s", cudaGetErrorString(ga));
       delete pl;
@@ -436,7 +472,26 @@ int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t*
     }
   // sizes, tables, planes
   const int oes = pl->i8 ? 1 : 2;
-  const int np = pl->i8 ? pl->max_slices : 2;
+  // FP64 by modular residues, as dense contractions: 14 exact products instead of
+  // the slices' 21, D updated once instead of six times, and a smaller error
+  // (1e-14 against 3e-14).  Not where a plan asks for slices, where the K blocks
+  // of an output block exceed one exact INT32 pass, or where the planes take too
+  // much memory.
+  if (pl->i8 && allow_residues && !(plan && (plan->slices > 0 || plan->moduli < 0))) {
+    int64_t kr = 1, kblocks = 1;
+    size_t in = 0, outb = 0;
+    for (auto* V : {&A, &B})
+      for (auto& o : *V) in += (size_t)rup(o.R, V == &B ? 256 : 128) * rup(o.K, 128);
+    for (auto& d : Ds) {
+      int64_t k = 0, b = 0;
+      for (auto& p : d.pairs) { k += A[p.first].K; b += rup(A[p.first].K, 128) / 128; }
+      kr = std::max(kr, k);
+      kblocks = std::max(kblocks, b);
+      outb += (size_t)rup(d.M, 128) * rup(d.N, 256);
+    }
+    pl->resid = kblocks <= kMaxPassBlocks && plan_residues(kr, 0, &pl->rp) && (in + outb) * pl->rp.rs.n <= kBscResidueBytes;
+  }
+  const int np = pl->resid ? pl->rp.rs.n : pl->i8 ? pl->max_slices : 2;
   std::vector<int64_t> tab;
   size_t plane_bytes = 0, erows = 0;
   int max_kb = 0;
@@ -468,14 +523,14 @@ int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t*
   }
   int err = 0;
   pl->tables = upload(pl, tab, &err, s);
-  pl->planes = (unsigned char*)dalloc(plane_bytes, &err);
+  pl->planes = (unsigned char*)dalloc(plane_bytes, &err, s);
   if (pl->planes) pl->allocs.push_back(pl->planes);
   pl->n_erows = erows;
-  pl->rowE = (unsigned*)dalloc(erows * sizeof(unsigned), &err);
+  pl->rowE = (unsigned*)dalloc(erows * sizeof(unsigned), &err, s);
   if (pl->rowE) pl->allocs.push_back(pl->rowE);
-  pl->rowexp = (int*)dalloc(erows * sizeof(int), &err);
+  pl->rowexp = (int*)dalloc(erows * sizeof(int), &err, s);
   if (pl->rowexp) pl->allocs.push_back(pl->rowexp);
-  pl->queue = (unsigned*)dalloc(sizeof(unsigned), &err);
+  pl->queue = (unsigned*)dalloc(sizeof(unsigned), &err, s);
   if (pl->queue) pl->allocs.push_back(pl->queue);
   if (err) { plan_free(pl); return err; }
   // gather jobs (A blocks, then B blocks) and their CTA maps
@@ -492,6 +547,7 @@ int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t*
       G.planes = pl->planes + o.plane_off;
       G.rowE = pl->rowE + o.e_off;
       G.slices = pl->slices;
+      if (pl->resid) G.rs = pl->rp.rs;
       G.lanes_on_k = (o.ks[0].s1 == 1 || o.rows[0].s1 != 1) ? 1 : 0;
       {  // 16-byte copies: whole groups of k that are contiguous and aligned in the block
         const int64_t vw = pl->i8 ? 2 : 4;
@@ -536,6 +592,20 @@ int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t*
   pl->dpair0.assign(Ds.size(), 0);
   pl->pair_maps.clear();
   int npairs = 0;
+  uint8_t* res = nullptr;
+  std::vector<size_t> res_off(Ds.size(), 0);
+  std::vector<CrtView> views;
+  std::vector<int2> crt_map;
+  if (pl->resid) {
+    size_t bytes = 0;
+    for (size_t d = 0; d < Ds.size(); ++d) {
+      res_off[d] = bytes;
+      bytes += (size_t)pl->rp.rs.n * rup(Ds[d].M, 128) * rup(Ds[d].N, 256);
+    }
+    res = (uint8_t*)dalloc(bytes, &err, s);
+    if (res) pl->allocs.push_back(res);
+    if (err) { plan_free(pl); return err; }
+  }
   for (size_t d = 0; d < Ds.size(); ++d) {
     dbl[d].D = Ds[d].ptr;
     dbl[d].dm = pl->tables + dm_off[d];
@@ -544,6 +614,14 @@ int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t*
     dbl[d].rowexp = pl->rowexp + A[Ds[d].pairs[0].first].e_off;
     dbl[d].colexp = pl->rowexp + B[Ds[d].pairs[0].second].e_off;
     dbl[d].M = (int)Ds[d].M; dbl[d].N = (int)Ds[d].N;
+    if (pl->resid) {
+      dbl[d].res = res + res_off[d];
+      dbl[d].res_ld = rup(Ds[d].N, 256);
+      dbl[d].res_plane = dbl[d].res_ld * rup(Ds[d].M, 128);
+      views.push_back({dbl[d].res, dbl[d].res_ld, dbl[d].res_plane, Ds[d].M, Ds[d].N, 1, 0, dbl[d].dm, dbl[d].dn, Ds[d].ptr,
+                       dbl[d].rowexp, dbl[d].colexp});
+      for (int64_t x = 0; x < crt_blocks(Ds[d].M, Ds[d].N, 1); ++x) crt_map.push_back(make_int2((int)d, (int)x));
+    }
     pl->dpair0[d] = npairs;
     for (auto& p : Ds[d].pairs) {
       pl->pair_maps.push_back(pl->maps + p.first);
@@ -553,15 +631,21 @@ int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t*
       ++npairs;
     }
   }
+  if (pl->resid) {
+    pl->crt_views = upload(pl, views, &err, s);
+    pl->crt_map = upload(pl, crt_map, &err, s);
+    pl->crt_ctas = (int64_t)crt_map.size();
+    if (pl->crt_ctas > INT32_MAX) { plan_free(pl); return TB_ERR_LIMIT; }
+  }
   {
     std::vector<BscPass> ps;
     std::vector<BscRun> rs;
     plan_passes(pl, pl->i8 ? pl->max_slices : 2, ps, rs, nullptr);  // the largest tables any slice count needs
     pl->passes_cap = ps.size();
     pl->runs_cap = rs.size();
-    pl->passes = (BscPass*)dalloc(ps.size() * sizeof(BscPass), &err);
+    pl->passes = (BscPass*)dalloc(ps.size() * sizeof(BscPass), &err, s);
     if (pl->passes) pl->allocs.push_back(pl->passes);
-    pl->runs = (BscRun*)dalloc(rs.size() * sizeof(BscRun), &err);
+    pl->runs = (BscRun*)dalloc(rs.size() * sizeof(BscRun), &err, s);
     if (pl->runs) pl->allocs.push_back(pl->runs);
   }
   pl->dblks = upload(pl, dbl, &err, s);
@@ -608,11 +692,13 @@ int bsc_prepare_attrs() {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(bsc_gemm_kernel<256, true, EPI_OZAKI_R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s256);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(bsc_gemm_kernel<128, false, EPI_BF16_R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s128);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(bsc_gemm_kernel<256, false, EPI_BF16_R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s256);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(bsc_gemm_kernel<128, true, EPI_RESID>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s128);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(bsc_gemm_kernel<256, true, EPI_RESID>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s256);
   if (e != cudaSuccess) { cudaGetLastError(); set_error("grouped GEMM attributes: %s", cudaGetErrorString(e)); return TB_ERR_CUDA; }
   return 0;
 }
 
-int kernels_per_run(const tb_bsc_plan_s* pl) { return pl->i8 ? 4 : 2; }
+int kernels_per_run(const tb_bsc_plan_s* pl) { return pl->resid ? 5 : pl->i8 ? 4 : 2; }
 
 // Captures the current configuration into a CUDA graph (on a private stream).
 int build_graph(tb_bsc_plan_s* pl) {
@@ -650,7 +736,10 @@ extern "C" int tb_bsc_plan_create(const char* pattern, int data_kind, int ntasks
   if (int e = bsc_prepare_attrs()) return e;
   tb_bsc_plan_s* pl = nullptr;
   int e = plan_create(pattern, data_kind, ntasks, tasks, alpha_real, alpha_imag, accumulative, plan, &pl,
-                      (cudaStream_t)stream);
+                      (cudaStream_t)stream, true);
+  if (e == TB_ERR_NO_MEMORY)  // without the residue planes
+    e = plan_create(pattern, data_kind, ntasks, tasks, alpha_real, alpha_imag, accumulative, plan, &pl,
+                    (cudaStream_t)stream, false);
   if (e) return e;
   *out = pl;
   return 0;
@@ -682,14 +771,14 @@ extern "C" int tb_bsc_autotune(tb_bsc_plan_t* pl, void* stream) {
   const int s0 = pl->slices, bn0 = pl->bn;
   pl->ar = 0.0; pl->ai = 0.0; pl->br = 1.0; pl->bi = 0.0;
   const int cand_s[2] = {6, 7};
-  const int ns = pl->i8 ? (pl->max_slices >= 7 ? 2 : 1) : 1;
+  const int ns = pl->i8 && !pl->resid ? (pl->max_slices >= 7 ? 2 : 1) : 1;
   float best = 1e30f;
   int bs = s0, bbn = bn0, err = 0;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   for (int si = 0; si < ns && !err; ++si) {
-    if (pl->i8 && (err = set_slices(pl, cand_s[si], s))) break;
+    if (pl->i8 && !pl->resid && (err = set_slices(pl, cand_s[si], s))) break;
     for (int bi2 = 0; bi2 < 2 && !err; ++bi2) {
       pl->bn = bi2 ? 256 : 128;
       if ((err = bsc_enqueue(pl, s))) break;  // warm-up
@@ -701,14 +790,14 @@ extern "C" int tb_bsc_autotune(tb_bsc_plan_t* pl, void* stream) {
       cudaEventElapsedTime(&ms, e0, e1);
       ms /= 2;
       pl->tune_ms[bi2][si] = ms;
-      if (ms < best) { best = ms; bs = pl->i8 ? cand_s[si] : s0; bbn = pl->bn; }
+      if (ms < best) { best = ms; bs = pl->i8 && !pl->resid ? cand_s[si] : s0; bbn = pl->bn; }
     }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   pl->ar = ar; pl->ai = ai; pl->br = br; pl->bi = bi;
   pl->bn = err ? bn0 : bbn;
-  if (pl->i8) {
+  if (pl->i8 && !pl->resid) {
     int e2 = set_slices(pl, err ? s0 : bs, s);
     if (!err) err = e2;
   }

@@ -21,6 +21,9 @@
 //            in a small shared-memory ring read by the other roles
 //   warp 1   TMEM allocation and the single MMA-issuing thread
 //   warps 2-5 epilogue
+// Residues: every modulus of an item is a work unit of its own (unit u: item u %
+// nitems, modulus u / nitems), since each writes its own plane; crt_grouped_kernel
+// then updates D once, where slices update it once per pass.
 // Every wait is bounded; one that gives up records its site in the device
 // error word: 11/12 producer (item slot, stage), 13/14/15 MMA issuer (item,
 // accumulator, stage), 16/17 epilogue (item, accumulator).
@@ -38,13 +41,16 @@ struct __align__(16) BscDBlk {  // output block
   int M, N;
   int pass0, npass;             // its accumulator passes: passes[pass0 .. pass0 + npass)
   int run0, nrun;               // its runs: runs[run0 .. run0 + nrun), pass after pass
+  uint8_t* res;                 // residues: its planes [modulus][row][column]
+  int64_t res_ld, res_plane;
 };
 struct BscItem { int d, mt, nt, pad_; };
 // A pass is one exact TMEM accumulator that the epilogue adds into the output
 // tile.  INT8 slices: its weight is 2^-shift; the operand blocks of one output
 // block share their row (column) scales, so products of several block pairs
 // add up exactly in INT32 within a pass.
-struct BscPass { int run0, nrun, shift, pad_; };
+// Residues: a pass is one modulus (shift; magic = floor(2^32 / shift)).
+struct BscPass { int run0, nrun, shift, magic; };
 // A run is what the producer streams without looking anything up: K blocks
 // [kb0, kb1) of plane a of one A block and plane b of one B block (tensor maps
 // for both N tiles).  The runs of an output block are flat, pass after pass;
@@ -68,6 +74,7 @@ struct __align__(64) BscParams {
   const BscRun* runs;
   unsigned int* queue;          // next item (zeroed before every launch)
   int nitems;
+  int moduli;                   // residues: work units are (item, modulus), moduli outermost; else 1
   double ar, ai, br, bi;        // beta applies to the first pass of each tile
   unsigned int* err;
 };
@@ -86,6 +93,20 @@ struct BscSmemBarriers {
 template <int BN>
 __host__ __device__ constexpr size_t bsc_smem_bytes() {
   return 1024 + (size_t)kStagesTC * (128 * 128 + BN * 128) + sizeof(BscSmemBarriers) + 64;
+}
+
+// The output block of a work unit; residues: reduced to the unit's pass.
+template <int EPI>
+__device__ __forceinline__ BscDBlk unit_block(const BscParams& P, int d, int unit) {
+  BscDBlk Dd = P.dblks[d];
+  if (EPI == EPI_RESID) {
+    Dd.pass0 += unit / P.nitems;
+    Dd.npass = 1;
+    const BscPass ps = P.passes[Dd.pass0];
+    Dd.run0 = ps.run0;
+    Dd.nrun = ps.nrun;
+  }
+  return Dd;
 }
 
 template <int BN, bool I8, int EPI>
@@ -122,13 +143,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) bsc_gemm_kernel(const __grid_co
       for (uint32_t k = 0; ok; ++k) {
         const int slot = (int)(k % kBscRing);
         if (!(ok = mbar_wait(&bars->item_empty[slot], ((k / kBscRing) & 1) ^ 1, P.err, 11u))) break;
-        const int item = (int)atomicAdd(P.queue, 1u);
-        const int cur = item < P.nitems ? item : -1;
+        const int unit = (int)atomicAdd(P.queue, 1u);
+        const int cur = unit < P.nitems * P.moduli ? unit : -1;
         bars->ring[slot] = cur;
         mbar_arrive(&bars->item_full[slot]);  // release: the ring entry is visible to the waiters
         if (cur < 0) break;
-        const BscItem I = P.items[cur];
-        const BscDBlk Dd = P.dblks[I.d];
+        const BscItem I = P.items[cur % P.nitems];
+        const BscDBlk Dd = unit_block<EPI>(P, I.d, cur);
         // software pipeline over the runs: the record of run r + 1 was loaded
         // during run r - 1 and its tensor maps are prefetched now; the record
         // of run r + 2 loads while run r streams
@@ -167,7 +188,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) bsc_gemm_kernel(const __grid_co
         if (!(ok = mbar_wait(&bars->item_full[slot], (k / kBscRing) & 1, P.err, 13u))) break;
         const int cur = bars->ring[slot];
         if (cur < 0) break;
-        const BscDBlk Dd = P.dblks[P.items[cur].d];
+        const BscDBlk Dd = unit_block<EPI>(P, P.items[cur % P.nitems].d, cur);
         const int rend = Dd.run0 + Dd.nrun;
         int2 ru = make_int2(0, 0), n1 = ru;  // (kb1 - kb0, flags) of runs r and r + 1
         {
@@ -220,22 +241,23 @@ __global__ void __launch_bounds__(kTcThreads, 1) bsc_gemm_kernel(const __grid_co
       if (!(ok = mbar_wait_warp(&bars->item_full[slot], (k / kBscRing) & 1, P.err, 16u))) break;
       const int cur = bars->ring[slot];
       if (cur < 0) break;
-      const BscItem I = P.items[cur];
-      const BscDBlk Dd = P.dblks[I.d];
+      const BscItem I = P.items[cur % P.nitems];
+      const BscDBlk Dd = unit_block<EPI>(P, I.d, cur);
       const int m = I.mt * 128 + quad * 32 + lane;
       const bool mval = m < Dd.M;
       const int64_t dmo = mval ? Dd.dm[m] : 0;
       // all pairs of an output block share its row and column scales
       const int re = (EPI == EPI_OZAKI_R) && mval ? Dd.rowexp[m] : 0;
-      const EpiView V{Dd.D, Dd.dn, Dd.colexp, Dd.N, P.ar, P.ai, P.br, P.bi, 0};
+      const EpiView V{Dd.D, Dd.dn, Dd.colexp, Dd.N, P.ar, P.ai, P.br, P.bi, 0, Dd.res};
       for (int p = Dd.pass0; p < Dd.pass0 + Dd.npass && ok; ++p, ++acc_it) {
         const int a = acc_it & 1;
         const uint32_t aph = (acc_it >> 1) & 1;
         if (!(ok = mbar_wait_warp(&bars->acc_full[a], aph, P.err, 17u, kEpilogueSleepNs))) break;
         tc_fence_after();
-        const int shift = (EPI == EPI_OZAKI_R) ? P.passes[p].shift : 0;
-        epilogue_pass<BN, EPI>(V, tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN), mval, dmo, re, I.nt,
-                               p == Dd.pass0, shift);
+        const int shift = (EPI == EPI_OZAKI_R || EPI == EPI_RESID) ? P.passes[p].shift : 0;
+        const int64_t off = EPI == EPI_RESID ? (int64_t)(cur / P.nitems) * Dd.res_plane + (int64_t)m * Dd.res_ld : dmo;
+        epilogue_pass<BN, EPI>(V, tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN), mval, off, re, I.nt,
+                               p == Dd.pass0, shift, EPI == EPI_RESID ? P.passes[p].magic : 0);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&bars->acc_empty[a]);

@@ -123,98 +123,6 @@ int launch_tc_epi(const TcGemmParams& P, int epi, bool pair, cudaStream_t s) {
   }
 }
 
-// ---- Ozaki scheme II: modular residues -----------------------------------------
-// Pairwise coprime moduli <= 256, largest first (their residues in the
-// symmetric range are signed 8-bit).  With n of them, M = prod m_i and the
-// operands scaled to integers |X| <= 2^p, an exact INT32 GEMM per modulus and
-// the Chinese remainder theorem give the exact integer product as long as
-// M > 2 Kr 2^(2p) (Kr: the real contraction length).
-constexpr int kModuliTable[kMaxModuli] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 211, 199, 197, 193};
-constexpr bool moduli_table_matches() {
-  for (int i = 0; i < kMaxModuli; ++i)
-    if (kModuliTable[i] != residue_modulus(i)) return false;
-  return true;
-}
-static_assert(moduli_table_matches(), "the gathers' compile-time moduli must be the plan's table");
-constexpr int kMinModuli = 8;
-constexpr int kMaxPassBlocks = 1023;  // K blocks of one exact INT32 pass (128^3 each, below 2^31)
-constexpr int kResidueBitsTarget = 46;  // operand bits kept by the default choice (INT8 slices keep 47)
-
-using u128 = unsigned __int128;
-
-u128 moduli_product(int n) {
-  u128 M = 1;
-  for (int i = 0; i < n; ++i) M *= (u128)kModuliTable[i];
-  return M;
-}
-
-// The largest p with M (1 - 2^-20) > 2 Kr 2^(2p) for n moduli (checked in exact
-// integer arithmetic; the 2^-20 is the room that crt_kernel's quotient needs).
-int residue_bits(int n, int64_t Kr) {
-  const u128 Mf = moduli_product(n), M = Mf - (Mf >> 20);
-  int p = 0;
-  while (p < 60 && (M >> (2 * (p + 1))) > (u128)(2 * Kr)) ++p;
-  return p;
-}
-
-struct ResiduePlan {
-  ResidueSpec rs;
-  int p;
-  CrtParams crt;  // constants only; pointers and sizes are filled by the caller
-};
-
-// Moduli count and constants for a contraction of real length Kr: `want` > 0
-// asks for that many moduli, else the fewest with p >= kResidueBitsTarget.
-// Returns false when no allowed count reaches kResidueBitsTarget bits.
-bool plan_residues(int64_t Kr, int want, ResiduePlan* out) {
-  int n = want;
-  if (n <= 0) {
-    for (n = kMinModuli; n <= kMaxModuli && residue_bits(n, Kr) < kResidueBitsTarget; ++n) {}
-    if (n > kMaxModuli) return false;
-  }
-  if (n < kMinModuli || n > kMaxModuli) return false;
-  // at most 52 bits: X = x 2^(p+1) rounded to an integer must be exact in
-  // FP64; the automatic choice keeps the 46-bit target (three 16-bit digits
-  // per operand in the gathers), an explicit moduli count all its bits
-  const int p = std::min(residue_bits(n, Kr), want > 0 ? 52 : kResidueBitsTarget);
-  if (p < 20) return false;
-  ResiduePlan& R = *out;
-  std::memset(&R, 0, sizeof(R));
-  R.p = p;
-  R.rs.n = n;
-  R.rs.pscale = std::ldexp(1.0, p + 1);
-  const u128 M = moduli_product(n);
-  R.crt.n = n;
-  R.crt.shift = 2 * (p + 1);
-  R.rs.p = p;
-  R.rs.ndig = p <= 46 ? 3 : 4;
-  int b = 0;
-  while (b < 127 && (M >> b) != 0) ++b;
-  // bits [b - 41 (k + 1), b - 41 k) of x, k = 0..2, as a double (exact)
-  auto part = [&](u128 x, int k) {
-    const int lo = std::max(0, b - 41 * (k + 1)), hi = std::max(0, b - 41 * k);
-    return std::ldexp((double)(uint64_t)((x >> lo) & (((u128)1 << (hi - lo)) - 1)), lo);
-  };
-  for (int i = 0; i < n; ++i) {
-    const int m = kModuliTable[i];
-    const u128 Mi = M / (u128)m;
-    const int mi_mod = (int)(Mi % (u128)m);
-    int y = 0;
-    for (int c = 1; c < m; ++c)
-      if ((mi_mod * c) % m == 1) { y = c; break; }
-    R.crt.mod[i] = m;
-    const u128 s = Mi * (u128)y;
-    R.crt.s1[i] = part(s, 0);
-    R.crt.s2[i] = part(s, 1);
-    R.crt.s3[i] = part(s, 2);
-  }
-  R.crt.M1 = part(M, 0);
-  R.crt.M2 = part(M, 1);
-  R.crt.M3 = part(M, 2);
-  R.crt.invM = 1.0 / (double)M;
-  return true;
-}
-
 }  // namespace
 
 int select_method(int dtk, const Matricization& Z, const tb_plan_t* plan) {
@@ -560,21 +468,12 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
     if (resid) {
       // Chinese remainder reconstruction of the exact products into D
       CrtParams C = RP.crt;
-      C.res = (const uint8_t*)(ws + offRES);
-      C.res_ld = Npad;
-      C.res_plane = Npad * Mpad;
-      C.rows = M;
-      C.cols = Nc;
-      C.dm = dm; C.dn = dn; C.D = d;
-      C.rowexp = rowx; C.colexp = colx;
+      C.v = {(const uint8_t*)(ws + offRES), Npad, Npad * Mpad, M, Nc, blocked ? kRowBlock : 1, 1, dm, dn, d, rowx, colx};
       C.ar = realpha; C.ai = cplx ? ai : 0.0; C.br = P.br; C.bi = 0.0;
-      C.row_step = blocked ? kRowBlock : 1;
-      const int64_t rb = (M + 32 * C.row_step - 1) / (32 * C.row_step) * C.row_step,
-                    cb = (Nr + kCrtCols * kCrtWarps - 1) / (kCrtCols * kCrtWarps);
-      if (rb * cb > INT32_MAX) { set_error("residue reconstruction grid too large"); err = TB_ERR_LIMIT; break; }
-      const unsigned cg = (unsigned)(rb * cb);
-      if (cplx) crt_kernel<true><<<cg, 32 * kCrtWarps, 0, s>>>(C);
-      else crt_kernel<false><<<cg, 32 * kCrtWarps, 0, s>>>(C);
+      const int64_t cg = crt_blocks(M, Nr, C.v.row_step);
+      if (cg > INT32_MAX) { set_error("residue reconstruction grid too large"); err = TB_ERR_LIMIT; break; }
+      if (cplx) crt_kernel<true><<<(unsigned)cg, 32 * kCrtWarps, 0, s>>>(C);
+      else crt_kernel<false><<<(unsigned)cg, 32 * kCrtWarps, 0, s>>>(C);
       count_launch();
       if (cudaError_t e = cudaGetLastError()) {
         set_error("residue reconstruction launch: %s", cudaGetErrorString(e));

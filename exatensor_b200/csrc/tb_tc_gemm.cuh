@@ -100,6 +100,7 @@ struct EpiView {
   int N;
   double ar, ai, br, bi;
   int nf_skip;
+  uint8_t* res;  // EPI_RESID: residue planes
 };
 
 // Ring through which the producer hands work units to the MMA and epilogue
@@ -166,7 +167,7 @@ __device__ __forceinline__ void epilogue_pass(const EP& P, uint32_t tcol, bool m
       // (!first) add their residue to the stored one.  With one byte store per
       // element this epilogue bounded K = 1600 products (102 us for 1600^2 x 15
       // moduli); packed it hides behind the next unit's MMAs.
-      if constexpr (std::is_same<EP, TcGemmParams>::value) {
+      {
         const uint32_t m = (uint32_t)shift, bias = ((0x80000000u + m - 1) / m) * m;
         auto residue = [&](uint32_t v) {
           v += bias;

@@ -835,20 +835,24 @@ __global__ void __launch_bounds__(256) nonfinite_fixup_kernel(const __grid_const
 // (four operations per residue) about alike.  A 60 KB shared-memory table of
 // 128-bit multiples, one random 16-byte read per residue, took 80 us for 1600^2
 // x 15 moduli and 2.6 ms for 36864 x 2304 x 14.
-struct CrtParams {
+struct CrtView {               // one output
   const uint8_t* res;          // residue planes [i][row][column], bytes
   int64_t res_ld, res_plane;
-  int n;
-  int mod[kMaxModuli];
-  double s1[kMaxModuli], s2[kMaxModuli], s3[kMaxModuli];
-  double M1, M2, M3, invM;
   int64_t rows, cols;          // rows of A; columns of B (complex: column pairs)
   int row_step;                // rows between a warp's lanes (blocked rows: the block, see TableJob)
+  int leave_flagged;           // 1: flagged rows and columns are the fix-up's; 0: they become NaN
   const int64_t* dm;
   const int64_t* dn;
   void* D;
   const int* rowexp;
   const int* colexp;
+};
+struct CrtParams {
+  CrtView v;                   // (dense form)
+  int n;
+  int mod[kMaxModuli];
+  double s1[kMaxModuli], s2[kMaxModuli], s3[kMaxModuli];
+  double M1, M2, M3, invM;
   int shift;                   // 2 (p + 1)
   double ar, ai, br, bi;
 };
@@ -859,27 +863,27 @@ struct CrtParams {
 constexpr int kCrtCols = 16, kCrtWarps = 4;
 
 template <bool CPLX>
-__global__ void __launch_bounds__(32 * kCrtWarps, 3) crt_kernel(const __grid_constant__ CrtParams P) {
+__device__ __forceinline__ void crt_body(const CrtParams& P, const CrtView& V, unsigned block) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned rs = (unsigned)P.row_step;
-  const unsigned row_blocks = (unsigned)((P.rows + 32 * rs - 1) / (32 * rs)) * rs;
-  const unsigned cb = blockIdx.x / row_blocks, rb = blockIdx.x - cb * row_blocks;
+  const unsigned rs = (unsigned)V.row_step;
+  const unsigned row_blocks = (unsigned)((V.rows + 32 * rs - 1) / (32 * rs)) * rs;
+  const unsigned cb = block / row_blocks, rb = block - cb * row_blocks;
   const int64_t m = ((int64_t)(rb / rs) * 32 + lane) * rs + rb % rs;
   constexpr int RC = CPLX ? 2 : 1, DC = kCrtCols / RC;  // residue columns per D column; D columns per thread
-  const int64_t rcols = P.cols * RC;
+  const int64_t rcols = V.cols * RC;
   const int64_t c0 = ((int64_t)cb * kCrtWarps + warp) * kCrtCols;
-  if (c0 >= rcols || m >= P.rows) return;
-  const int re = P.rowexp[m];
-  if (re >= kNonFiniteExp) return;  // flagged row: the fix-up's
-  const uint8_t* rp = P.res + m * P.res_ld + c0;  // rows are padded to whole column tiles: always inside the plane
+  if (c0 >= rcols || m >= V.rows) return;
+  const int re = V.rowexp[m];
+  if (re >= kNonFiniteExp && V.leave_flagged) return;  // flagged row: the fix-up's
+  const uint8_t* rp = V.res + m * V.res_ld + c0;  // rows are padded to whole column tiles: always inside the plane
   uint4 w[kMaxModuli];
 #pragma unroll
   for (int i = 0; i < kMaxModuli; ++i)
-    w[i] = i < P.n ? *reinterpret_cast<const uint4*>(rp + i * P.res_plane) : make_uint4(0, 0, 0, 0);
-  const int64_t dmo = P.dm[m];
+    w[i] = i < P.n ? *reinterpret_cast<const uint4*>(rp + i * V.res_plane) : make_uint4(0, 0, 0, 0);
+  const int64_t dmo = V.dm[m];
   const bool read_d = P.br != 0.0 || P.bi != 0.0;
   using E = typename std::conditional<CPLX, double2, double>::type;
-  E* D = (E*)P.D;
+  E* D = (E*)V.D;
   constexpr int G = 8, H = G / RC;  // residue columns and D columns of one group
 #pragma unroll
   for (int g = 0; g < kCrtCols / G; ++g) {
@@ -890,10 +894,10 @@ __global__ void __launch_bounds__(32 * kCrtWarps, 3) crt_kernel(const __grid_con
     for (int j = 0; j < H; ++j) {
       const int64_t n = c0 / RC + g * H + j;
       o[j] = -1;
-      if (n >= P.cols) continue;
-      ce[j] = P.colexp[n * RC];
-      if (ce[j] >= kNonFiniteExp) continue;  // flagged column: the fix-up's
-      o[j] = dmo + P.dn[n];
+      if (n >= V.cols) continue;
+      ce[j] = V.colexp[n * RC];
+      if (ce[j] >= kNonFiniteExp && V.leave_flagged) continue;  // flagged column: the fix-up's
+      o[j] = dmo + V.dn[n];
       if (read_d) old[j] = D[o[j]];
     }
     double a[G], b[G], c[G];
@@ -918,6 +922,7 @@ __global__ void __launch_bounds__(32 * kCrtWarps, 3) crt_kernel(const __grid_con
       const double x = fma(-Q, P.M1, a[j]), y = fma(-Q, P.M2, b[j]), z = fma(-Q, P.M3, c[j]);  // exact
       const double t = x + y, yy = t - x;
       const double err = (x - (t - yy)) + (y - yy);  // x + y = t + err exactly
+      if (re >= kNonFiniteExp || cexp >= kNonFiniteExp) return __longlong_as_double(0x7FF8000000000000ll);
       return scale2(t + (err + z), re + cexp - P.shift);
     };
 #pragma unroll
@@ -939,6 +944,118 @@ __global__ void __launch_bounds__(32 * kCrtWarps, 3) crt_kernel(const __grid_con
       }
     }
   }
+}
+
+template <bool CPLX>
+__global__ void __launch_bounds__(32 * kCrtWarps, 3) crt_kernel(const __grid_constant__ CrtParams P) {
+  crt_body<CPLX>(P, P.v, blockIdx.x);
+}
+
+// Grouped form: CTA x works on block map[x].y of output map[x].x.
+__global__ void __launch_bounds__(32 * kCrtWarps, 3) crt_grouped_kernel(const __grid_constant__ CrtParams P,
+                                                                       const CrtView* __restrict__ outputs,
+                                                                       const int2* __restrict__ map) {
+  const int2 jm = map[blockIdx.x];
+  const CrtView V = outputs[jm.x];
+  crt_body<false>(P, V, (unsigned)jm.y);
+}
+
+// CTAs of one output.
+int64_t crt_blocks(int64_t rows, int64_t residue_cols, int row_step) {
+  return (rows + 32 * row_step - 1) / (32 * row_step) * row_step *
+         ((residue_cols + kCrtCols * kCrtWarps - 1) / (kCrtCols * kCrtWarps));
+}
+
+// ---- Ozaki scheme II: the plan ------------------------------------------------------
+// Pairwise coprime moduli <= 256, largest first (their residues in the
+// symmetric range are signed 8-bit).  With n of them, M = prod m_i and the
+// operands scaled to integers |X| <= 2^p, an exact INT32 GEMM per modulus and
+// the Chinese remainder theorem give the exact integer product as long as
+// M > 2 Kr 2^(2p) (Kr: the real contraction length).
+constexpr int kModuliTable[kMaxModuli] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 211, 199, 197, 193};
+constexpr bool moduli_table_matches() {
+  for (int i = 0; i < kMaxModuli; ++i)
+    if (kModuliTable[i] != residue_modulus(i)) return false;
+  return true;
+}
+static_assert(moduli_table_matches(), "the gathers' compile-time moduli must be the plan's table");
+constexpr int kMinModuli = 8;
+constexpr int kMaxPassBlocks = 1023;  // K blocks of one exact INT32 pass (128^3 each, below 2^31)
+constexpr int kResidueBitsTarget = 46;  // operand bits kept by the default choice (INT8 slices keep 47)
+
+using u128 = unsigned __int128;
+
+u128 moduli_product(int n) {
+  u128 M = 1;
+  for (int i = 0; i < n; ++i) M *= (u128)kModuliTable[i];
+  return M;
+}
+
+// The largest p with M (1 - 2^-20) > 2 Kr 2^(2p) for n moduli (checked in exact
+// integer arithmetic; the 2^-20 is the room that crt_kernel's quotient needs).
+int residue_bits(int n, int64_t Kr) {
+  const u128 Mf = moduli_product(n), M = Mf - (Mf >> 20);
+  int p = 0;
+  while (p < 60 && (M >> (2 * (p + 1))) > (u128)(2 * Kr)) ++p;
+  return p;
+}
+
+struct ResiduePlan {
+  ResidueSpec rs;
+  int p;
+  CrtParams crt;  // constants only; pointers and sizes are filled by the caller
+};
+
+// Moduli count and constants for a contraction of real length Kr: `want` > 0
+// asks for that many moduli, else the fewest with p >= kResidueBitsTarget.
+// Returns false when no allowed count reaches kResidueBitsTarget bits.
+bool plan_residues(int64_t Kr, int want, ResiduePlan* out) {
+  int n = want;
+  if (n <= 0) {
+    for (n = kMinModuli; n <= kMaxModuli && residue_bits(n, Kr) < kResidueBitsTarget; ++n) {}
+    if (n > kMaxModuli) return false;
+  }
+  if (n < kMinModuli || n > kMaxModuli) return false;
+  // at most 52 bits: X = x 2^(p+1) rounded to an integer must be exact in
+  // FP64; the automatic choice keeps the 46-bit target (three 16-bit digits
+  // per operand in the gathers), an explicit moduli count all its bits
+  const int p = std::min(residue_bits(n, Kr), want > 0 ? 52 : kResidueBitsTarget);
+  if (p < 20) return false;
+  ResiduePlan& R = *out;
+  std::memset(&R, 0, sizeof(R));
+  R.p = p;
+  R.rs.n = n;
+  R.rs.pscale = std::ldexp(1.0, p + 1);
+  const u128 M = moduli_product(n);
+  R.crt.n = n;
+  R.crt.shift = 2 * (p + 1);
+  R.rs.p = p;
+  R.rs.ndig = p <= 46 ? 3 : 4;
+  int b = 0;
+  while (b < 127 && (M >> b) != 0) ++b;
+  // bits [b - 41 (k + 1), b - 41 k) of x, k = 0..2, as a double (exact)
+  auto part = [&](u128 x, int k) {
+    const int lo = std::max(0, b - 41 * (k + 1)), hi = std::max(0, b - 41 * k);
+    return std::ldexp((double)(uint64_t)((x >> lo) & (((u128)1 << (hi - lo)) - 1)), lo);
+  };
+  for (int i = 0; i < n; ++i) {
+    const int m = kModuliTable[i];
+    const u128 Mi = M / (u128)m;
+    const int mi_mod = (int)(Mi % (u128)m);
+    int y = 0;
+    for (int c = 1; c < m; ++c)
+      if ((mi_mod * c) % m == 1) { y = c; break; }
+    R.crt.mod[i] = m;
+    const u128 s = Mi * (u128)y;
+    R.crt.s1[i] = part(s, 0);
+    R.crt.s2[i] = part(s, 1);
+    R.crt.s3[i] = part(s, 2);
+  }
+  R.crt.M1 = part(M, 0);
+  R.crt.M2 = part(M, 1);
+  R.crt.M3 = part(M, 2);
+  R.crt.invM = 1.0 / (double)M;
+  return true;
 }
 
 // Row maxima of the FP64 exponent fields (the slice scales), streamed without
