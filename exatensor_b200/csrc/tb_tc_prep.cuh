@@ -870,36 +870,47 @@ __device__ __forceinline__ void crt_body(const CrtParams& P, const CrtView& V, u
   const unsigned cb = block / row_blocks, rb = block - cb * row_blocks;
   const int64_t m = ((int64_t)(rb / rs) * 32 + lane) * rs + rb % rs;
   constexpr int RC = CPLX ? 2 : 1, DC = kCrtCols / RC;  // residue columns per D column; D columns per thread
-  const int64_t rcols = V.cols * RC;
   const int64_t c0 = ((int64_t)cb * kCrtWarps + warp) * kCrtCols;
-  if (c0 >= rcols || m >= V.rows) return;
-  const int re = V.rowexp[m];
-  if (re >= kNonFiniteExp && V.leave_flagged) return;  // flagged row: the fix-up's
-  const uint8_t* rp = V.res + m * V.res_ld + c0;  // rows are padded to whole column tiles: always inside the plane
+  if (c0 >= V.cols * RC) return;
+  const bool mok = m < V.rows;
+  // Everything that depends on nothing is loaded at once, so that a warp waits for
+  // two memory latencies, not five: its row's exponent and D offset, its columns'
+  // (one column per lane, handed around by shuffles), its residues; then D.
+  const int re = mok ? V.rowexp[m] : kNonFiniteExp;
+  const int64_t dmo = mok ? V.dm[m] : 0;
+  const int64_t nl = c0 / RC + (lane < DC ? lane : 0);
+  const bool lok = nl < V.cols;
+  const int ce_l = lok ? V.colexp[nl * RC] : kNonFiniteExp;
+  const int64_t dn_l = lok ? V.dn[nl] : 0;
+  const uint8_t* rp = V.res + (mok ? m : 0) * V.res_ld + c0;  // rows are padded to whole column tiles: always inside the plane
   uint4 w[kMaxModuli];
 #pragma unroll
   for (int i = 0; i < kMaxModuli; ++i)
     w[i] = i < P.n ? *reinterpret_cast<const uint4*>(rp + i * V.res_plane) : make_uint4(0, 0, 0, 0);
-  const int64_t dmo = V.dm[m];
   const bool read_d = P.br != 0.0 || P.bi != 0.0;
   using E = typename std::conditional<CPLX, double2, double>::type;
   E* D = (E*)V.D;
-  constexpr int G = 8, H = G / RC;  // residue columns and D columns of one group
+  constexpr int G = 8, H = G / RC, NG = kCrtCols / G;  // residue columns and D columns of one group
+  // column j of D: its offset (-1: not written here) and exponent
+  auto column = [&](int j, int64_t& o, int& ce) {
+    ce = __shfl_sync(0xffffffffu, ce_l, j);
+    const int64_t dn = __shfl_sync(0xffffffffu, dn_l, j);
+    const bool in = mok && c0 / RC + j < V.cols;
+    const bool flagged = re >= kNonFiniteExp || ce >= kNonFiniteExp;
+    o = in && !(flagged && V.leave_flagged) ? dmo + dn : -1;
+  };
+  E old[NG][H];
 #pragma unroll
-  for (int g = 0; g < kCrtCols / G; ++g) {
-    E old[H];
-    int64_t o[H];
-    int ce[H];
+  for (int g = 0; g < NG; ++g)
 #pragma unroll
     for (int j = 0; j < H; ++j) {
-      const int64_t n = c0 / RC + g * H + j;
-      o[j] = -1;
-      if (n >= V.cols) continue;
-      ce[j] = V.colexp[n * RC];
-      if (ce[j] >= kNonFiniteExp && V.leave_flagged) continue;  // flagged column: the fix-up's
-      o[j] = dmo + V.dn[n];
-      if (read_d) old[j] = D[o[j]];
+      int64_t o;
+      int ce;
+      column(g * H + j, o, ce);
+      if (read_d && o >= 0) old[g][j] = D[o];
     }
+#pragma unroll
+  for (int g = 0; g < NG; ++g) {
     double a[G], b[G], c[G];
 #pragma unroll
     for (int j = 0; j < G; ++j) a[j] = b[j] = c[j] = 0.0;
@@ -927,20 +938,23 @@ __device__ __forceinline__ void crt_body(const CrtParams& P, const CrtView& V, u
     };
 #pragma unroll
     for (int j = 0; j < H; ++j) {
-      if (o[j] < 0) continue;
+      int64_t o;
+      int ce;
+      column(g * H + j, o, ce);
+      if (o < 0) continue;
       if constexpr (!CPLX) {
-        const double v = P.ar * combine(j, ce[j]);
-        D[o[j]] = P.br == 0.0 ? v : fma(P.br, old[j], v);
+        const double v = P.ar * combine(j, ce);
+        D[o] = P.br == 0.0 ? v : fma(P.br, old[g][j], v);
       } else {
-        const double xr = combine(2 * j, ce[j]), xi = combine(2 * j + 1, ce[j]);
+        const double xr = combine(2 * j, ce), xi = combine(2 * j + 1, ce);
         double2 v;
         v.x = P.ar * xr - P.ai * xi;
         v.y = P.ar * xi + P.ai * xr;
         if (read_d) {
-          v.x += P.br * old[j].x - P.bi * old[j].y;
-          v.y += P.br * old[j].y + P.bi * old[j].x;
+          v.x += P.br * old[g][j].x - P.bi * old[g][j].y;
+          v.y += P.br * old[g][j].y + P.bi * old[g][j].x;
         }
-        D[o[j]] = v;
+        D[o] = v;
       }
     }
   }
