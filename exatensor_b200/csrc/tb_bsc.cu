@@ -145,7 +145,7 @@ int bsc_enqueue(tb_bsc_plan_s* pl, cudaStream_t s) {
                                                                                                        pl->rm_map);
     TB_CHECK_LAUNCH();
     exps_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)(pl->n_erows + 255) / 256, 4096)), 256, 0,
-                  s>>>(pl->rowE, pl->rowexp, (int64_t)pl->n_erows, 1);
+                  s>>>(pl->rowE, pl->rowexp, (int64_t)pl->n_erows);
     TB_CHECK_LAUNCH();
   }
   // the gathers read the slice count from the jobs: keep them in sync with the configuration
@@ -570,8 +570,10 @@ int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t*
   pl->rm_ctas = (int64_t)rm_map.size();
   pl->g_ctas = (int64_t)g_map.size();
   const int64_t want = (int64_t)num_sms() * 16;
-  pl->rm_gy = (int)std::max<int64_t>(1, std::min<int64_t>(max_kt, want / std::max<int64_t>(1, pl->rm_ctas)));
-  pl->g_gy = (int)std::max<int64_t>(1, std::min<int64_t>(max_kt, want / std::max<int64_t>(1, pl->g_ctas)));
+  // uneven blocks: K tiles are dealt to at least four (two) CTAs per row tile, so
+  // that the largest blocks do not end last
+  pl->rm_gy = (int)std::min<int64_t>(max_kt, std::max<int64_t>(4, want / std::max<int64_t>(1, pl->rm_ctas)));
+  pl->g_gy = (int)std::min<int64_t>(max_kt, std::max<int64_t>(2, want / std::max<int64_t>(1, pl->g_ctas)));
   if (pl->rm_ctas > INT32_MAX || pl->g_ctas > INT32_MAX) { plan_free(pl); return TB_ERR_LIMIT; }
   // tensor maps: A (128-row boxes), B for BN = 128 and 256
   std::vector<CUtensorMap> maps((size_t)A.size() + 2 * B.size());

@@ -161,7 +161,17 @@ int plan_direct(const Matricization& Z, int es, bool cplx, const void* d, const 
     for (int box = 0; box < 2; ++box) {
       if (force_box >= 0 && box != force_box) continue;
       int tp = 1, tq = 1;
-      double mrows = (double)cdiv(M, sh.bm) * sh.bm, amp = pm == 0 || P.a_on_k || M == 1 ? 1.0 : sector;
+      double mrows = (double)cdiv(M, sh.bm) * sh.bm, amp = 1.0;
+      if (pm > 0) {
+        // linear rows still hold runs of the contiguous group when few rows of
+        // the groups before it fill less than a tile; L1 serves their sectors
+        double before = 1.0;
+        for (int i = 0; i < pm; ++i) before *= (double)m[i].ext;
+        const double run = std::max(1.0, std::min((double)m[pm].ext, sh.bm / before));
+        amp = std::min(sector, (run * es + 32.0 - es) / (run * es));
+      } else if (pm < 0 && !P.a_on_k && M > 1) {
+        amp = sector;
+      }
       if (box) {
         if (pm <= 0 || sh.bm < 32) continue;
         // the box with the least traffic: runs of tp (operand) and tq (D)

@@ -703,19 +703,16 @@ cudaError_t gather_grouped_prepare() {
   return smem_limit_once(once, gather_grouped_kernel<MODE>, gather_smem_bytes<MODE>());
 }
 
-// exponents: rowexp[r] = rowE[r / rep] - 1021 (rep = 2 for complex B' rows).
-// With a list, the source rows flagged 2047 (a NaN or an infinity) are also
-// appended to it (in no particular order; *count counts them).
-__global__ void exps_kernel(const unsigned* __restrict__ rowE, int* __restrict__ out, int64_t n, int rep,
-                            int* __restrict__ list = nullptr, int* __restrict__ count = nullptr) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const unsigned e = rowE[i / rep];
-    out[i] = (int)e - 1021;
-    if (list && e >= 2047u && i % rep == 0) list[atomicAdd(count, 1)] = (int)(i / rep);
-  }
+// exponents: rowexp[r] = rowE[r] - 1021
+__global__ void exps_kernel(const unsigned* __restrict__ rowE, int* __restrict__ out, int64_t n) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = (int)rowE[i] - 1021;
 }
 
-// Both operands' exponents in one launch.
+// Both operands' exponents in one launch: rowx[r] = rowE[r] - 1021, colx likewise
+// (rep = 2 for complex B' rows).  Rows and columns flagged 2047 (a NaN or an
+// infinity) are also appended to the bad lists (in no particular order; nbad[0..1]
+// count them).
 __global__ void exps_pair_kernel(const unsigned* __restrict__ rowE, int* __restrict__ rowx, int64_t m,
                                  int* __restrict__ badrows, const unsigned* __restrict__ colE, int* __restrict__ colx,
                                  int64_t n, int rep, int* __restrict__ badcols, int* __restrict__ nbad) {
@@ -832,9 +829,10 @@ __global__ void __launch_bounds__(256) nonfinite_fixup_kernel(const __grid_const
 // + f_n - 2(p+1)) exactly, and D = beta D + alpha C through the offset tables.
 // Rows and columns flagged as holding a NaN or an infinity are left to the
 // fix-up kernel.  Bound by the bytes of the planes and D and by the FP64 units
-// (four operations per residue) about alike.  A 60 KB shared-memory table of
-// 128-bit multiples, one random 16-byte read per residue, took 80 us for 1600^2
-// x 15 moduli and 2.6 ms for 36864 x 2304 x 14.
+// (four operations per residue) about alike, and for small outputs by its memory
+// latencies: 40 us for 1600^2 x 15 moduli, 68 us for 9216 x 576 x 15.  A 60 KB
+// shared-memory table of 128-bit multiples, one random 16-byte read per residue, took
+// 80 and 161 us.
 struct CrtView {               // one output
   const uint8_t* res;          // residue planes [i][row][column], bytes
   int64_t res_ld, res_plane;
@@ -1140,7 +1138,10 @@ __device__ __forceinline__ void rowmax_body(const GatherParams& P, int64_t rowti
   for (int it = 0; it < IT; ++it) {
     const int idx = tid + it * kGThreads;
     const int mm = idx / TK;
-    if (emax[it]) atomicMax(&sm_max[mm], emax[it]);
+    // the lanes of a warp hold one row: one atomic per warp and row instead of 32 on
+    // one shared word (the 40^6 product's row maxima: 36 -> 27 us)
+    const unsigned e = __reduce_max_sync(0xffffffffu, emax[it]);
+    if ((tid & 31) == 0 && e) atomicMax(&sm_max[mm], e);
   }
   __syncthreads();
   if (tid < TM && sm_max[tid] && m0 + tid < P.rows) atomicMax(&P.rowE[m0 + tid], sm_max[tid]);

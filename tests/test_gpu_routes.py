@@ -1,0 +1,66 @@
+"""Where TB_METHOD_AUTO sends FP64 products, and the operand orders of the
+tensor-core path.
+
+Long R8 and C8 products that the selector leaves to the plain method run with
+15 moduli; short ones in one kernel.  Tolerance of the former: operands keep 51
+bits (2^-51 each, relative to a row's largest value, about 1.7 times the rms of
+uniform data) and the FP64 reference itself carries about sqrt(K) 2^-54.
+
+The fused path's rows run in blocks of eight of the left operand's contiguous
+group when D's fastest group is another one: groups shorter than a block, whole
+blocks, and blocks with a remainder."""
+import numpy as np
+import pytest
+import torch
+
+import exatensor_b200 as XB
+import oracle as O
+from tests.test_gpu_contract import oracle_dd
+from tests.test_gpu_permute import rand_host
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind,dt,m,n,k,moduli", [(XB.R8, torch.float64, 1400, 1100, 1290, 15),
+                                                  (XB.C8, torch.complex128, 900, 700, 1000, 15),
+                                                  (XB.R8, torch.float64, 1300, 1200, 200, 0)])
+def test_long_products_keep_51_bits(xt, dev, kind, dt, m, n, k, moduli):
+    g = torch.Generator(device="cuda").manual_seed(k)
+    real = torch.float64
+    mk = lambda *s: (torch.rand(*s, dtype=real, device="cuda", generator=g) * 2 - 1)  # noqa: E731
+    l, r, d = [mk(*s) if dt == real else torch.complex(mk(*s), mk(*s)) for s in ((m, k), (n, k), (n, m))]
+    want = r @ l.T + d  # D(i,j), i fastest; L(k,i) and R(k,j) with k fastest
+    plain = np.zeros(16 * 8 + 8 + 64 + 8 + 8 * XB.SELECT_PLANS + XB.SELECT_PLANS, np.float32)
+    plain[-XB.SELECT_PLANS + 1:] = 9.0
+    # a caller's network that picks the plain method keeps it: one kernel, no residues
+    XB.selector_install(8, plain, np.zeros(16, np.float32), np.ones(16, np.float32))
+    try:
+        out = d.clone()
+        xt.tensor_contract("D(i,j)+=L(k,i)*R(k,j)", kind, [m, n], out.data_ptr(), [k, m], l.data_ptr(), [k, n],
+                           r.data_ptr(), 1.0, stream=torch.cuda.current_stream())
+        st = xt.last_contract_stats()
+        assert st.method == XB.METHOD_TTGT and st.moduli == 0
+        assert (torch.linalg.norm(out - want) / torch.linalg.norm(want)).item() <= 4e-15
+    finally:
+        XB.selector_install(0, None, None, None)
+    out = d.clone()
+    # below the size rule's 4e9 operations: picked plain, then refined
+    xt.tensor_contract("D(i,j)+=L(k,i)*R(k,j)", kind, [m, n], out.data_ptr(), [k, m], l.data_ptr(), [k, n], r.data_ptr(),
+                       1.0, stream=torch.cuda.current_stream())
+    st = xt.last_contract_stats()
+    assert st.moduli == moduli and (not moduli or st.residue_bits >= 51)
+    assert (torch.linalg.norm(out - want) / torch.linalg.norm(want)).item() <= 4e-15
+
+
+@pytest.mark.parametrize("dtk,tol", [(O.R8, 1e-12), (O.C8, 1e-12), (O.R4, 1e-4), (O.C4, 1e-4)])
+@pytest.mark.parametrize("c", [3, 8, 19, 24])
+def test_blocked_rows(xt, dev, dtk, tol, c):
+    pattern, ext = "D(a,b,c,d)+=L(c,k,a,l)*R(l,d,k,b)", dict(a=9, b=5, c=c, d=7, k=6, l=40)
+    ddims, ldims, rdims = [[ext[x] for x in g] for g in ("abcd", "ckal", "ldkb")]
+    d, l, r = [rand_host(dtk, int(np.prod(x)), 3 + i) for i, x in enumerate((ddims, ldims, rdims))]
+    ref = oracle_dd(pattern, d, ddims, l, ldims, r, rdims, 0.5, True)
+    dd, ld, rd = dev.put(d), dev.put(l), dev.put(r)
+    xt.tensor_contract(pattern, dtk, ddims, dd.data_ptr(), ldims, ld.data_ptr(), rdims, rd.data_ptr(), 0.5,
+                       plan=xt.make_plan(XB.METHOD_FUSED), stream=dev.stream())
+    assert O.rel_frobenius(dev.get(dd, d.dtype, d.size), ref) <= tol
+    xt.device_check(dev.stream())
