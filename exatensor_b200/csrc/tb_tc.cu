@@ -218,14 +218,22 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
   const int64_t K = Z.K;
   const int64_t Kr = cplx ? 2 * K : K, Nr = cplx ? 2 * Nc : Nc;
   const int64_t Kpad = round_up(Kr, 128);
-  const int BN = (plan && plan->tile_n == 128) ? 128 : (plan && plan->tile_n == 256) ? 256 : (Nr >= 192 ? 256 : 128);
+  // N tile: what the plan asks for, else 256 (128 for narrow products).  The residue
+  // GEMM is bound by the bytes that its tiles read from L2 (128 + BN rows of 128 bytes
+  // per K block), so without a request it takes 192 where that reads a twelfth less:
+  // N = 576 in three tiles of 192 instead of three of 256 (9216 x 576 x 9216 by 15
+  // moduli: 1589 -> 1553 us in all).
+  const bool asks_tile = plan && (plan->tile_n == 128 || plan->tile_n == 256);
+  int BN = asks_tile ? plan->tile_n : Nr >= 192 ? 256 : 128;
+  if (!asks_tile && i8 && !(plan && (plan->slices > 0 || plan->moduli < 0 || plan->tile_m == 256)) && Nr > 128 &&
+      12 * ((Nr + 191) / 192) * (128 + 192) <= 11 * ((Nr + 255) / 256) * (128 + 256))
+    BN = 192;
   // M tile: one SM per 128-row tile unless the plan asks for SM pairs (256
   // rows); the pair kernel halves the B traffic per SM but measured no faster
   // on the CCSD-like shapes, whose GEMMs run at the power cap.
   const bool pair = plan && plan->tile_m == 256;
   const int TM = pair ? 256 : 128;
-  const int64_t Mpad = round_up(M, TM), Npad = round_up(Nr, BN);
-  if (Mpad / 128 * (Npad / BN) > INT32_MAX || M > INT32_MAX || Nr > INT32_MAX) return TB_ERR_LIMIT;
+  const int64_t Mpad = round_up(M, TM);
   // products and passes: an entry multiplies plane a of A by plane b of B over
   // a K-block range; the entries of a pass share one exact INT32 accumulator.
   struct Entry { int a, b, kb0, kb1; };
@@ -245,6 +253,9 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
     set_error("modular residues: %d moduli do not fit this contraction (K = %lld)", plan->moduli, (long long)Kr);
     return TB_ERR_INVALID_ARGS;
   }
+  if (!resid && BN == 192) BN = 256;  // residues only
+  const int64_t Npad = round_up(Nr, BN);
+  if (Mpad / 128 * (Npad / BN) > INT32_MAX || M > INT32_MAX || Nr > INT32_MAX) return TB_ERR_LIMIT;
   if (resid) {
     const int chunk = (kblocks + res_nch - 1) / res_nch;
     for (int i = 0; i < RP.rs.n; ++i)
@@ -462,7 +473,9 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
     P.l2hint = hint_env >= 0 ? (hint_env ? 1 : 0) : (resid && bplane <= (size_t)96 << 20 ? 1 : 0);
     const int epi = resid ? EPI_RESID : i8 ? (cplx ? EPI_OZAKI_C : EPI_OZAKI_R) : (cplx ? EPI_BF16_C : EPI_BF16_R);
     const int ts = timed_begin(s);
-    err = BN == 256 ? launch_tc_epi<256>(P, epi, pair, s) : launch_tc_epi<128>(P, epi, pair, s);
+    err = BN == 256   ? launch_tc_epi<256>(P, epi, pair, s)
+          : BN == 192 ? launch_tc<192, true, EPI_RESID>(P, s)
+                      : launch_tc_epi<128>(P, epi, pair, s);
     timed_end(ts, s);
     if (err) break;
     if (resid) {

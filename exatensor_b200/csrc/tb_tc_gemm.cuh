@@ -277,6 +277,7 @@ __device__ __forceinline__ void epilogue_pass(const EP& P, uint32_t tcol, bool m
 template <int BN, bool I8, int EPI>
 __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_constant__ TcGemmParams P) {
   using namespace sm100;
+  constexpr int kAccCols = BN == 192 ? 256 : BN;  // TMEM columns of an accumulator (allocations are powers of two)
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* smA = base;                                    // [stages][128 rows][128 B]
@@ -297,7 +298,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
     prefetch_tmap(&P.tmB);
   }
   if (warp == 1) {
-    tmem_alloc(&bars->tmem_base, 2 * BN);
+    tmem_alloc(&bars->tmem_base, 2 * kAccCols);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -373,7 +374,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
           const uint32_t aph = (acc_it >> 1) & 1;
           if (!(ok = mbar_wait(&bars->acc_empty[a], aph ^ 1, P.err))) break;
           tc_fence_after();
-          const uint32_t dcol = tmem + (uint32_t)(a * BN);
+          const uint32_t dcol = tmem + (uint32_t)(a * kAccCols);
           bool first = true;
           for (int q = P.pass_first[p]; q < P.pass_first[p + 1] && ok; ++q) {
             for (int kb = P.prod_kb0[q]; kb < P.prod_kb1[q]; ++kb, ++it) {
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
         const bool first = EPI == EPI_RESID ? (p - w.p0 == 0) : (p == 0);
         const int shift = (EPI == EPI_OZAKI_R || EPI == EPI_OZAKI_C || EPI == EPI_RESID) ? P.pass_shift[p] : 0;
         const int64_t dmp = EPI == EPI_RESID ? (int64_t)(p / P.res_nch) * P.res_plane + (int64_t)m * P.res_ld : dmo;
-        epilogue_pass<BN, EPI>(P, tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * BN),
+        epilogue_pass<BN, EPI>(P, tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(a * kAccCols),
                                mval, dmp, re, nb, first, shift,
                                EPI == EPI_RESID ? P.pass_magic[p] : 0);
         tc_fence_before();
@@ -429,7 +430,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, 2 * BN);
+    tmem_dealloc(tmem, 2 * kAccCols);
   }
 }
 

@@ -64,3 +64,20 @@ def test_blocked_rows(xt, dev, dtk, tol, c):
                        plan=xt.make_plan(XB.METHOD_FUSED), stream=dev.stream())
     assert O.rel_frobenius(dev.get(dd, d.dtype, d.size), ref) <= tol
     xt.device_check(dev.stream())
+
+
+@pytest.mark.parametrize("kind,n,tile", [(XB.R8, 129, 192), (XB.R8, 192, 192), (XB.R8, 193, 256), (XB.R8, 575, 192),
+                                         (XB.C8, 190, 192), (XB.C8, 65, 192), (XB.R8, 128, 128)])
+def test_residue_tile_of_192_columns(xt, dev, kind, n, tile):
+    """The N tile of residue products without a request, at its edges (complex
+    products have 2n real columns); same tolerance as 14 moduli elsewhere."""
+    m, k = 200, 300
+    g = torch.Generator(device="cuda").manual_seed(n)
+    mk = lambda *s: (torch.rand(*s, dtype=torch.float64, device="cuda", generator=g) * 2 - 1)  # noqa: E731
+    l, r, d = [mk(*s) if kind == XB.R8 else torch.complex(mk(*s), mk(*s)) for s in ((m, k), (n, k), (n, m))]
+    want = r @ l.T + d
+    xt.tensor_contract("D(i,j)+=L(k,i)*R(k,j)", kind, [m, n], d.data_ptr(), [k, m], l.data_ptr(), [k, n], r.data_ptr(),
+                       1.0, plan=xt.make_plan(XB.METHOD_FUSED), stream=torch.cuda.current_stream())
+    assert xt.last_contract_stats().tile_n == tile
+    assert (torch.linalg.norm(d - want) / torch.linalg.norm(want)).item() <= 1e-13
+    xt.device_check(dev.stream())
