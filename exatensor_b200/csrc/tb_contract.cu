@@ -371,12 +371,15 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
     auto refine = [&](int picked, bool callers, int* err) {
       const bool asked = plan && (plan->slices || plan->tile_n || plan->tile_m || plan->bf16_terms || plan->moduli);
       if (picked == TB_METHOD_FUSED && (asked || callers)) return false;
+      // What the one-kernel form declines keeps the picked method: an output that
+      // overlaps an operand is multiplied from copies (TTGT), and for more groups
+      // than its parameter block holds nothing predicts the plain method's time.
       DirectPlan dp;
-      const bool direct_ok = direct_plan(Z, dtk, d, l, r, &dp) == 0;
+      if (direct_plan(Z, dtk, d, l, r, &dp) != 0) return false;
       const int64_t Kr = cplx ? 2 * Z.K : Z.K;
       constexpr int64_t kExactMinK = 256;
       if (picked == TB_METHOD_TTGT && is_double(dtk) && !callers && !asked && Kr >= kExactMinK &&
-          predicted_fused_us(Z, dtk, 15) < (direct_ok ? dp.us : 1e30)) {
+          predicted_fused_us(Z, dtk, 15) < dp.us) {
         tb_plan_t rp{};
         rp.method = TB_METHOD_FUSED;
         rp.moduli = 15;
@@ -389,7 +392,6 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
           return true;
         }
       }
-      if (!direct_ok) return false;
       if (picked == TB_METHOD_FUSED && dp.us >= predicted_fused_us(Z, dtk, 14)) return false;
       g_stats.method = TB_METHOD_TTGT;
       g_stats.gemm_launches = 1;

@@ -81,3 +81,48 @@ def test_residue_tile_of_192_columns(xt, dev, kind, n, tile):
     assert xt.last_contract_stats().tile_n == tile
     assert (torch.linalg.norm(d - want) / torch.linalg.norm(want)).item() <= 1e-13
     xt.device_check(dev.stream())
+
+
+def test_output_over_an_operand_is_multiplied_from_copies(xt, dev):
+    """D starts inside L, and L's infinity lies where another row of D goes: the
+    product still sees the old L.  (The infinity's row is infinite, other entries are
+    sums of 300 FP64 products and an accumulated old element.)"""
+    m, n, k, off = 96, 80, 300, 3
+    rng = np.random.default_rng(4)
+    x = rng.uniform(-1, 1, k * m + n * m + off)
+    x[5] = np.inf  # L(5, 0); also D(2, 0)
+    r = rng.uniform(-1, 1, n * k)
+    lm, rm, d0 = x[:k * m].reshape(k, m), r.reshape(k, n), x[off:off + n * m].reshape(n, m)
+    with np.errstate(invalid="ignore"):
+        want = rm.T @ lm + d0
+    buf, rd = dev.put(x), dev.put(r)
+    xt.tensor_contract("D(a,b)+=L(a,k)*R(b,k)", XB.R8, [m, n], buf.data_ptr() + 8 * off, [m, k], buf.data_ptr(), [n, k],
+                       rd.data_ptr(), 1.0, stream=dev.stream())
+    st = xt.last_contract_stats()
+    got = dev.get(buf, np.float64)[off:off + n * m].reshape(n, m)
+    assert np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    fin = np.isfinite(want)
+    assert fin.sum() >= (m - 2) * n and np.array_equal(np.isfinite(got), fin)
+    assert np.linalg.norm(got[fin] - want[fin]) <= 4e-15 * np.linalg.norm(want[fin])
+    assert st.method == XB.METHOD_TTGT and st.moduli == 0
+
+
+def test_more_groups_than_the_one_kernel_form_holds(xt, dev):
+    """14 free indices of extent 2 in an order that nothing merges: the plain method runs, not residues."""
+    rank, k = 14, 300
+    a = "abcdefghijlmno"[:rank]
+    perm = list(range(0, rank, 2)) + list(range(1, rank, 2))
+    pattern = "D(%s,z)+=L(k,%s)*R(k,z)" % (",".join(a), ",".join(a[i] for i in perm))
+    rng = np.random.default_rng(5)
+    l, r = rng.uniform(-1, 1, k << rank), rng.uniform(-1, 1, 3 * k)
+    dd, ld, rd = dev.put(np.zeros(3 << rank)), dev.put(l), dev.put(r)
+    xt.tensor_contract(pattern, XB.R8, [2] * rank + [3], dd.data_ptr(), [k] + [2] * rank, ld.data_ptr(), [k, 3],
+                       rd.data_ptr(), 1.0, accumulative=False, stream=dev.stream())
+    st = xt.last_contract_stats()
+    assert st.method == XB.METHOD_TTGT and st.moduli == 0
+    # numpy's axes run the other way round
+    lt = l.reshape([2] * rank + [k])            # axes: index perm[rank-1], ..., perm[0], k
+    c = np.tensordot(r.reshape(3, k), lt, axes=([1], [rank]))  # z, perm[rank-1], ..., perm[0]
+    axis = {perm[rank - 1 - i]: i + 1 for i in range(rank)}
+    want = c.transpose([0] + [axis[rank - 1 - i] for i in range(rank)]).ravel()
+    assert np.linalg.norm(dev.get(dd, np.float64) - want) <= 4e-15 * np.linalg.norm(want)
