@@ -359,10 +359,14 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
     //    to 30 us instead of 27 to 100 us for small ones).
     //  * R8 and C8 products picked plain but long enough run as residues with 15
     //    moduli, 51 or 52 operand bits, where that is predicted faster: 96/24
-    //    ladder 4.04 -> 1.59 ms, 1600^3 475 -> 210 us.  Their error is below the
-    //    plain sums' from K = 256 on (relative to long double, uniform data: 5e-17
-    //    against 5e-16 at K = 256, 1.3e-15 at 1600; normal data 4e-16 against 5e-16
-    //    and 1.4e-15), because nothing rounds inside a sum.
+    //    ladder 4.04 -> 1.57 ms, 1600^3 475 -> 186 us.  Residues keep those bits relative to
+    //    a row's largest value, not of every element, so the GPU first counts how far
+    //    the rows' values spread (GuardParams): where residues could be off by more
+    //    than the bound of the FP64 sum, as with magnitudes that fall along the
+    //    contracted index or many zeros, it runs the one-kernel form instead, for the
+    //    price of the counting pass (96/24 ladder 0.16 ms).  Measured relative to long double:
+    //    uniform data 5e-17 against the plain sums' 5e-16 at K = 256 and 1.3e-15 at
+    //    1600; normal data 4e-16 against 5e-16 and 1.4e-15.
     //  * A product picked for the tensor cores runs in one kernel where that is
     //    predicted faster than their preparation alone (K = 9856, M = N = 150: 147
     //    us against 67 us).
@@ -376,16 +380,15 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
       // than its parameter block holds nothing predicts the plain method's time.
       DirectPlan dp;
       if (direct_plan(Z, dtk, d, l, r, &dp) != 0) return false;
-      const int64_t Kr = cplx ? 2 * Z.K : Z.K;
       constexpr int64_t kExactMinK = 256;
-      if (picked == TB_METHOD_TTGT && is_double(dtk) && !callers && !asked && Kr >= kExactMinK &&
+      if (picked == TB_METHOD_TTGT && is_double(dtk) && !callers && !asked && Z.K >= kExactMinK &&
           predicted_fused_us(Z, dtk, 15) < dp.us) {
         tb_plan_t rp{};
         rp.method = TB_METHOD_FUSED;
         rp.moduli = 15;
         const int fe = contract_fused(Z, dtk, ddims, d, ldims, l, rdims, r, ar, ai, accumulative != 0, lconj, rconj, &rp,
-                                      s, &g_stats);
-        // short of scratch, or K beyond the pass table: as before
+                                      s, &g_stats, &dp);
+        // short of scratch, or K too long for 51 bits: as before
         if (fe != TB_ERR_NO_MEMORY && fe != TB_ERR_NOT_IMPLEMENTED && fe != TB_ERR_LIMIT && fe != TB_ERR_INVALID_ARGS) {
           g_stats.method = TB_METHOD_FUSED;
           *err = fe;

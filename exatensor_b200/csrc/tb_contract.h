@@ -7,6 +7,8 @@
 
 namespace tb {
 
+struct DirectPlan;
+
 int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* d, int lrank, const int* ldims,
                   const void* l, int rrank, const int* rdims, const void* r, double ar, double ai, int conj_bits,
                   int accumulative, const tb_plan_t* plan, cudaStream_t s);
@@ -16,9 +18,12 @@ int select_method(int dtk, const Matricization& Z, const tb_plan_t* plan);
 
 // Tensor-core contraction with fused operand gathers and epilogue.
 // Returns TB_ERR_NOT_IMPLEMENTED when the shape is outside its scope.
+// `otherwise` (R8, C8 by residues): the GPU looks at the operands' magnitudes and runs
+// this one-kernel form instead where residues may lose against FP64 sums; not
+// implemented where fewer than 51 bits per operand fit.
 int contract_fused(const Matricization& Z, int dtk, const int* ddims, void* d, const int* ldims, const void* l,
                    const int* rdims, const void* r, double ar, double ai, bool accumulate, int lconj, int rconj,
-                   const tb_plan_t* plan, cudaStream_t s, tb_contract_stats_t* stats);
+                   const tb_plan_t* plan, cudaStream_t s, tb_contract_stats_t* stats, const DirectPlan* otherwise = nullptr);
 
 // Predicted microseconds of contract_fused's default plan (R8, C8: n moduli).
 double predicted_fused_us(const Matricization& Z, int dtk, int n);

@@ -20,8 +20,15 @@ struct Variant {
   using S = Shape<E, WM, WN, KW, MI, NI, BK, ST>;
   static TileShape shape() { return {S::BM, S::BN, S::BKT, S::T, OCC}; }
   static int launch(const Params& P, int64_t ctas, cudaStream_t s) {
+    if constexpr (!Elem<E>::F32) {  // conditional launches: FP64 data only
+      if (P.when) return launch_as<true>(P, ctas, s);
+    }
+    return launch_as<false>(P, ctas, s);
+  }
+  template <bool WHEN>
+  static int launch_as(const Params& P, int64_t ctas, cudaStream_t s) {
     static DeviceOnce attr;
-    auto kern = direct_kernel<E, WM, WN, KW, MI, NI, BK, ST, OCC>;
+    auto kern = direct_kernel<E, WM, WN, KW, MI, NI, BK, ST, OCC, WHEN>;
     const size_t smem = S::smem(P.split > 1 || KW > 1);
     cudaError_t e = smem_limit_once(attr, kern, (int)S::smem(true));
     if (e != cudaSuccess) { set_error("direct contraction smem attribute: %s", cudaGetErrorString(e)); return TB_ERR_CUDA; }
@@ -110,8 +117,9 @@ int direct_plan(const Matricization& Z, int dtk, const void* d, const void* l, c
 }
 
 int run_direct(const DirectPlan& plan, int dtk, double ar, double ai, bool accumulate, int lconj, int rconj,
-               cudaStream_t s) {
+               cudaStream_t s, const unsigned* when) {
   Params P = plan.P;
+  P.when = when;
   P.ar = ar;
   P.ai = ai;
   P.br = accumulate ? 1.0 : 0.0;

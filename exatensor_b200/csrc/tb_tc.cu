@@ -31,6 +31,7 @@
 
 #include "tb_common.cuh"
 #include "tb_contract.h"
+#include "tb_direct.h"
 #include "tb_permute.cuh"
 #include "tb_tc_gemm.cuh"
 #include "tb_tc_prep.cuh"
@@ -169,7 +170,7 @@ double predicted_fused_us(const Matricization& Z, int dtk, int n) {
 
 int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, const int* ldims, const void* l,
                    const int* rdims, const void* r, double ar, double ai, bool accumulate, int lconj, int rconj,
-                   const tb_plan_t* plan, cudaStream_t s, tb_contract_stats_t* stats) {
+                   const tb_plan_t* plan, cudaStream_t s, tb_contract_stats_t* stats, const DirectPlan* otherwise) {
   (void)ddims;
   if (Z0.K < 1 || Z0.M < 1 || Z0.N < 1 || Z0.k.empty()) return TB_ERR_NOT_IMPLEMENTED;
   Matricization Z = Z0;
@@ -253,6 +254,7 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
     set_error("modular residues: %d moduli do not fit this contraction (K = %lld)", plan->moduli, (long long)Kr);
     return TB_ERR_INVALID_ARGS;
   }
+  if (otherwise && (!resid || RP.p < 51 || Kr > 65535)) return TB_ERR_NOT_IMPLEMENTED;
   if (!resid && BN == 192) BN = 256;  // residues only
   const int64_t Npad = round_up(Nr, BN);
   if (Mpad / 128 * (Npad / BN) > INT32_MAX || M > INT32_MAX || Nr > INT32_MAX) return TB_ERR_LIMIT;
@@ -339,7 +341,10 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
                offKB = offKA + al(K * 8), offRE = offKB + al(K * 8), offCE = offRE + al(M * 4),
                offNB = offCE + al(Nc * 4), offRX = offNB + 256, offCX = offRX + al(M * 4), offBR = offCX + al(Nr * 4),
                offBC = offBR + al(M * 4), offRES = offBC + al(Nc * 4),
-               total = offRES + (resid ? al((size_t)RP.rs.n * Npad * Mpad) : 0);
+               offSA = offRES + (resid ? al((size_t)RP.rs.n * Npad * Mpad) : 0);
+  const int splitsA = !otherwise ? 0 : cplx ? rowmax_splits<true>(M, K) : rowmax_splits<false>(M, K);
+  const int splitsB = !otherwise ? 0 : cplx ? rowmax_splits<true>(Nc, K) : rowmax_splits<false>(Nc, K);
+  const size_t offSB = offSA + al(sizeof(RowSpread) * splitsA * M), total = offSB + al(sizeof(RowSpread) * splitsB * Nc);
   unsigned char* ws = nullptr;
   if (int e = scratch_alloc((void**)&ws, total, s)) return e;
   int err = 0;
@@ -357,7 +362,8 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
   int* colx = (int*)(ws + offCX);
   int* badrows = (int*)(ws + offBR);  // rows of A / columns of B holding a NaN or an infinity
   int* badcols = (int*)(ws + offBC);
-  int* nbad = (int*)(ws + offNB);
+  int* nbad = (int*)(ws + offNB);     // counts of both, the GEMM's work-unit counter, GuardParams::words from nbad[8] on
+  const unsigned* refused = otherwise ? (const unsigned*)nbad + 15 : nullptr;
   const int64_t ksrc_pad = cplx ? Kpad / 2 : Kpad;  // padded K in source elements
   do {
     // Offset tables and cleared words (row maxima, counters) in one launch.  A's
@@ -407,23 +413,39 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
     // holding a NaN or an infinity (exponent field 2047): the epilogue leaves
     // their D entries to nonfinite_fixup_kernel.  nbad[0..1]: flagged row /
     // column counts; nbad[2]: the GEMM's work-unit counter.
+    GuardParams GP{};
+    if (otherwise) {
+      GA.spread = (RowSpread*)(ws + offSA);
+      GB.spread = (RowSpread*)(ws + offSB);
+      GP.a = GA.spread; GP.b = GB.spread;
+      GP.m = M; GP.n = Nc;
+      GP.gy_a = splitsA; GP.gy_b = splitsB;
+      GP.kr = (int)Kr;
+      for (int i = 1; i <= 3; ++i) GP.need[i - 1] = std::max(1 << (55 + 2 * i - RP.p), (int)((Kr + 3) / 4));
+      GP.words = (unsigned*)nbad + 8;
+    }
     auto run_exps = [&]() -> int {
-      exps_pair_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((M + Nr + 255) / 256, 4096)), 256, 0, s>>>(
-          rowE, rowx, M, badrows, colE, colx, Nr, cplx ? 2 : 1, badcols, nbad);
+      // GUARD: eight lanes per row
+      const int64_t items = otherwise ? 8 * (M + Nc) : M + Nr;
+      const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((items + 255) / 256, otherwise ? 4 * num_sms() : 4096));
+      if (otherwise)
+        exps_pair_kernel<true><<<grid, 256, 0, s>>>(rowE, rowx, M, badrows, colE, colx, Nr, cplx ? 2 : 1, badcols, nbad, GP);
+      else
+        exps_pair_kernel<false><<<grid, 256, 0, s>>>(rowE, rowx, M, badrows, colE, colx, Nr, cplx ? 2 : 1, badcols, nbad, GP);
       TB_CHECK_LAUNCH();
       return 0;
     };
     if (i8) {
       if ((err = cplx ? run_rowmax<true>(GA, GB, s) : run_rowmax<false>(GA, GB, s))) break;
       if ((err = run_exps())) break;
-      if (resid) err = cplx ? run_gather<G_RESID_C8A, G_RESID_C8B>(GA, GB, gA, gB, gk, s)
-                            : run_gather<G_RESID_R8, G_RESID_R8>(GA, GB, gA, gB, gk, s);
-      else err = cplx ? run_gather<G_SLICE_C8A, G_SLICE_C8B>(GA, GB, gA, gB, gk, s)
-                      : run_gather<G_SLICE_R8, G_SLICE_R8>(GA, GB, gA, gB, gk, s);
+      if (resid) err = cplx ? run_gather<G_RESID_C8A, G_RESID_C8B>(GA, GB, gA, gB, gk, refused, s)
+                            : run_gather<G_RESID_R8, G_RESID_R8>(GA, GB, gA, gB, gk, refused, s);
+      else err = cplx ? run_gather<G_SLICE_C8A, G_SLICE_C8B>(GA, GB, gA, gB, gk, refused, s)
+                      : run_gather<G_SLICE_R8, G_SLICE_R8>(GA, GB, gA, gB, gk, refused, s);
       if (err) break;
     } else {
-      if ((err = cplx ? run_gather<G_SPLIT_C4A, G_SPLIT_C4B>(GA, GB, gA, gB, gk, s)
-                      : run_gather<G_SPLIT_R4, G_SPLIT_R4>(GA, GB, gA, gB, gk, s)))
+      if ((err = cplx ? run_gather<G_SPLIT_C4A, G_SPLIT_C4B>(GA, GB, gA, gB, gk, refused, s)
+                      : run_gather<G_SPLIT_R4, G_SPLIT_R4>(GA, GB, gA, gB, gk, refused, s)))
         break;
       if ((err = run_exps())) break;  // the split gathers flag non-finite rows
     }
@@ -455,6 +477,7 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
     P.ar = realpha; P.ai = cplx ? ai : 0.0;
     P.br = accumulate ? 1.0 : 0.0; P.bi = 0.0;
     P.err = device_error_word();
+    P.refused = refused;
     P.nf_skip = resid ? 0 : 1;  // residues: crt_kernel leaves the flagged entries to the fix-up
     if (resid) {
       P.res = (uint8_t*)(ws + offRES);
@@ -483,6 +506,7 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
       CrtParams C = RP.crt;
       C.v = {(const uint8_t*)(ws + offRES), Npad, Npad * Mpad, M, Nc, blocked ? kRowBlock : 1, 1, dm, dn, d, rowx, colx};
       C.ar = realpha; C.ai = cplx ? ai : 0.0; C.br = P.br; C.bi = 0.0;
+      C.refused = refused;
       const int64_t cg = crt_blocks(M, Nr, C.v.row_step);
       if (cg > INT32_MAX) { set_error("residue reconstruction grid too large"); err = TB_ERR_LIMIT; break; }
       if (cplx) crt_kernel<true><<<(unsigned)cg, 32 * kCrtWarps, 0, s>>>(C);
@@ -503,6 +527,7 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
     F.rowE = rowE; F.badrows = badrows; F.badcols = badcols; F.nbad = nbad;
     F.isignA = A.conj ? -1.0 : 1.0; F.isignB = B.conj ? -1.0 : 1.0;
     F.ar = realpha; F.ai = cplx ? ai : 0.0; F.br = P.br; F.bi = 0.0;
+    F.refused = refused;
     const unsigned fgrid = (unsigned)(2 * num_sms());
     if (dtk == kR8) nonfinite_fixup_kernel<double, false><<<fgrid, 256, 0, s>>>(F);
     else if (dtk == kC8) nonfinite_fixup_kernel<double, true><<<fgrid, 256, 0, s>>>(F);
@@ -514,6 +539,7 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
       err = TB_ERR_CUDA;
       break;
     }
+    if (otherwise && (err = run_direct(*otherwise, dtk, realpha, cplx ? ai : 0.0, accumulate, lconj, rconj, s, refused))) break;
     if (stats) {
       stats->slices = S;
       stats->passes = (int)passes.size();

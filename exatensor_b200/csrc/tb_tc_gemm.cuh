@@ -61,6 +61,7 @@ struct __align__(64) TcGemmParams {
   int64_t res_ld, res_plane;  // EPI_RESID: row stride and plane stride (bytes)
   int res_nch;                // EPI_RESID: passes per modulus (K chunks of at most
                               // 1023 blocks each, added up mod m by the epilogue)
+  const unsigned int* refused;  // nothing to do if this word is set (null: never; single-SM kernel)
   unsigned int* sched;        // single-SM kernel: zeroed work-unit counter (dynamic
                               // scheduling), or null for a static round robin
   int l2hint;                 // 1: A tiles are loaded evict-first and B tiles
@@ -277,6 +278,7 @@ __device__ __forceinline__ void epilogue_pass(const EP& P, uint32_t tcol, bool m
 template <int BN, bool I8, int EPI>
 __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_constant__ TcGemmParams P) {
   using namespace sm100;
+  if (P.refused && *P.refused) return;
   constexpr int kAccCols = BN == 192 ? 256 : BN;  // TMEM columns of an accumulator (allocations are powers of two)
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)tc_smem_raw + 1023) & ~(uintptr_t)1023);

@@ -216,6 +216,29 @@ struct ResidueSpec {
   int ndig;                 // balanced 16-bit digits of X: 3 (p <= 46) or 4
 };
 
+// How a row's values spread below its largest: bits 16 j .. 16 j + 15 of `bins` count
+// the values with exponent field e - j, j = 0..3 (of use for e > 3 only: field 0 holds
+// zeros and subnormal values); e is 0 only for a row of zeros.
+struct __align__(16) RowSpread {
+  unsigned long long bins;
+  unsigned e, pad_;
+};
+__device__ __forceinline__ void spread_add(RowSpread& S, double x) {
+  const unsigned f = exp_field(x);
+  if (f > S.e || S.e == 0) {  // seldom, but for the first values
+    const unsigned g = f ? f : (x != 0.0 ? 1u : 0u), up = g - S.e;
+    S.bins = up > 3 ? 0ull : S.bins << (16 * up);
+    S.e = g;
+  }
+  const unsigned j = S.e - f;
+  S.bins += j <= 3 ? 1ull << (16 * j) : 0ull;
+}
+__device__ __forceinline__ void spread_merge(RowSpread& S, const RowSpread& o) {
+  const unsigned e = max(S.e, o.e), a = e - S.e, b = e - o.e;
+  S.bins = (a > 3 ? 0ull : S.bins << (16 * a)) + (b > 3 ? 0ull : o.bins << (16 * b));
+  S.e = e;
+}
+
 struct GatherParams {
   const void* src;
   const int64_t* lm;   // source offset of row m (m < rows)
@@ -226,6 +249,7 @@ struct GatherParams {
   void* planes;
   unsigned* rowE;      // per row: largest exponent field (slice modes read it; the
                        // split modes set it to 2047 for rows with a NaN or an infinity)
+  RowSpread* spread;   // row maxima that also count: [K split][row]; else null
   int slices;
   int lanes_on_k;      // 1: consecutive k are contiguous in the source
   int vec;             // 1 (lanes_on_k): aligned 16-byte groups of k are contiguous and aligned in the source
@@ -668,12 +692,14 @@ struct GatherPair {
   GatherParams a, b;
   unsigned ctas_a, rows_a, rows_b;
   int gy_a, gy_b;
+  const unsigned* refused;  // nothing to do if this word is set (null: never)
 };
 
 // (the complex residue modes leave two CTAs per SM registers enough not to spill)
 template <int MODEA, int MODEB, int NDIG = 3>
 __global__ void __launch_bounds__(kGThreads, MODEB == G_RESID_C8B ? 2 : 3)
     gather_kernel(const __grid_constant__ GatherPair Q) {
+  if (Q.refused && *Q.refused) return;
   const bool second = blockIdx.x >= Q.ctas_a;
   const unsigned x = second ? blockIdx.x - Q.ctas_a : blockIdx.x, rows = second ? Q.rows_b : Q.rows_a;
   const unsigned ky = x / rows, rt = x - ky * rows;
@@ -709,13 +735,35 @@ __global__ void exps_kernel(const unsigned* __restrict__ rowE, int* __restrict__
     out[i] = (int)rowE[i] - 1021;
 }
 
+// Whether residues may stand for FP64 sums, decided from the operands.  With p
+// operand bits a residue product is off by at most K 2^(a + b + 2 - p), 2^a and 2^b the
+// binades of the row's and the column's largest values.  If at least C of the K pairs
+// hold two values within s binades of those, the sum of |products| is at least C 2^(a +
+// b - 2 s), so that bound is K 2^(2 + 2 s - p) / C of it, and no larger than the K 2^-53
+// of a sum of K FP64 terms where C >= 2^(55 + 2 s - p).  C is at least K minus the
+// values of the worst row and of the worst column that are not within s binades;
+// C >= K / 4 is asked for as well.  Rows and columns with a NaN or an infinity (the
+// fix-up multiplies them in FP64) and rows of zeros do not count.
+struct GuardParams {
+  const RowSpread* a;        // [K split][row] of both operands
+  const RowSpread* b;
+  int64_t m, n;              // rows, columns
+  int gy_a, gy_b;            // K splits
+  int kr;                    // values per row
+  int need[3];               // C for s = 1, 2, 3
+  unsigned* words;           // zeroed: [0..2], [3..5] values missing in the worst row and column, [6]
+                             // CTAs done, [7] the verdict: 1 where residues are refused
+};
+
 // Both operands' exponents in one launch: rowx[r] = rowE[r] - 1021, colx likewise
 // (rep = 2 for complex B' rows).  Rows and columns flagged 2047 (a NaN or an
 // infinity) are also appended to the bad lists (in no particular order; nbad[0..1]
-// count them).
-__global__ void exps_pair_kernel(const unsigned* __restrict__ rowE, int* __restrict__ rowx, int64_t m,
+// count them).  GUARD: the last CTA writes the verdict.
+template <bool GUARD>
+__global__ void __launch_bounds__(256) exps_pair_kernel(const unsigned* __restrict__ rowE, int* __restrict__ rowx, int64_t m,
                                  int* __restrict__ badrows, const unsigned* __restrict__ colE, int* __restrict__ colx,
-                                 int64_t n, int rep, int* __restrict__ badcols, int* __restrict__ nbad) {
+                                 int64_t n, int rep, int* __restrict__ badcols, int* __restrict__ nbad,
+                                 const __grid_constant__ GuardParams G) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m + n; i += (int64_t)gridDim.x * blockDim.x) {
     const bool col = i >= m;
     const int64_t j = col ? i - m : i;
@@ -724,6 +772,51 @@ __global__ void exps_pair_kernel(const unsigned* __restrict__ rowE, int* __restr
     if (e >= 2047u) {
       if (!col) badrows[atomicAdd(nbad, 1)] = (int)j;
       else if (j % rep == 0) badcols[atomicAdd(nbad + 1, 1)] = (int)(j / rep);
+    }
+  }
+  if constexpr (GUARD) {
+    // eight lanes merge a row's records
+    unsigned miss[2][3] = {{0, 0, 0}, {0, 0, 0}};
+    const int lane = threadIdx.x & 31, sub = lane & 7;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); 4 * w < G.m + G.n; w += warps) {
+      const int64_t i = 4 * w + (lane >> 3);
+      const bool in = i < G.m + G.n, col = i >= G.m;
+      const int64_t r = col ? i - G.m : i, rows = col ? G.n : G.m;
+      RowSpread S{0ull, 0u, 0u};
+      if (in)
+#pragma unroll 4
+        for (int y = sub; y < (col ? G.gy_b : G.gy_a); y += 8) spread_merge(S, ((col ? G.b : G.a) + y * rows)[r]);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        const RowSpread T{__shfl_xor_sync(0xffffffffu, S.bins, o), __shfl_xor_sync(0xffffffffu, S.e, o), 0u};
+        spread_merge(S, T);
+      }
+      if (S.e == 0 || S.e >= 2047u) continue;
+      if (S.e <= 3) S.bins = 0;
+      int c = G.kr - (int)(S.bins & 0xFFFF);
+#pragma unroll
+      for (int s = 0; s < 3; ++s) {
+        c -= (int)((S.bins >> (16 * (s + 1))) & 0xFFFF);
+        if (col) miss[1][s] = max(miss[1][s], (unsigned)c);
+        else miss[0][s] = max(miss[0][s], (unsigned)c);
+      }
+    }
+#pragma unroll
+    for (int o = 0; o < 2; ++o)
+#pragma unroll
+      for (int s = 0; s < 3; ++s) {
+        const unsigned v = __reduce_max_sync(0xffffffffu, miss[o][s]);
+        if (lane == 0 && v) atomicMax(&G.words[3 * o + s], v);
+      }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&G.words[6], 1u) == gridDim.x - 1) {
+      __threadfence();
+      bool ok = false;
+      for (int s = 0; s < 3; ++s)
+        ok = ok || G.kr - (int)atomicAdd(&G.words[s], 0u) - (int)atomicAdd(&G.words[3 + s], 0u) >= G.need[s];
+      G.words[7] = ok ? 0u : 1u;
     }
   }
 }
@@ -751,12 +844,14 @@ struct NfParams {
   const int* nbad;
   double isignA, isignB;                  // -1: conjugate the operand
   double ar, ai, br, bi;                  // alpha, beta (beta 0: D is not read)
+  const unsigned* refused;                // nothing to do if this word is set (null: never)
 };
 
 template <typename R, bool CPLX>
 __global__ void __launch_bounds__(256) nonfinite_fixup_kernel(const __grid_constant__ NfParams P) {
   const int nbr = P.nbad[0], nbc = P.nbad[1];
   if (nbr == 0 && nbc == 0) return;
+  if (P.refused && *P.refused) return;
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   const int64_t total = (int64_t)nbr * P.N + (int64_t)nbc * P.M;
@@ -853,6 +948,7 @@ struct CrtParams {
   double M1, M2, M3, invM;
   int shift;                   // 2 (p + 1)
   double ar, ai, br, bi;
+  const unsigned* refused;     // nothing to do if this word is set (null: never)
 };
 
 // A warp takes 32 rows (lanes; D's fastest) and a thread kCrtCols residue
@@ -960,6 +1056,7 @@ __device__ __forceinline__ void crt_body(const CrtParams& P, const CrtView& V, u
 
 template <bool CPLX>
 __global__ void __launch_bounds__(32 * kCrtWarps, 3) crt_kernel(const __grid_constant__ CrtParams P) {
+  if (P.refused && *P.refused) return;
   crt_body<CPLX>(P, P.v, blockIdx.x);
 }
 
@@ -1073,17 +1170,28 @@ bool plan_residues(int64_t Kr, int want, ResiduePlan* out) {
 // Row maxima of the FP64 exponent fields (the slice scales), streamed without
 // shared-memory staging: each thread keeps the running maximum of the rows it
 // touches in registers over all K tiles of its CTA, and the CTA merges them once
-// at the end.  Thread -> (row, k) mapping as in gather_kernel.
-template <bool CPLX>
+// at the end.  Thread -> (row, k) mapping as in gather_kernel.  SPREAD: the same
+// for a RowSpread per row, written per CTA (P.spread).
+template <bool CPLX, bool SPREAD>
 __device__ __forceinline__ void rowmax_body(const GatherParams& P, int64_t rowtile, int ky, int kstep) {
   using E = typename std::conditional<CPLX, double2, double>::type;
   constexpr int TM = gather_rows<E>(), TK = kGK, IT = TM * TK / kGThreads;
   __shared__ unsigned sm_max[TM];
+  __shared__ RowSpread sm_spread[SPREAD ? kGThreads : 1];
   const int tid = threadIdx.x;
   if (tid < TM) sm_max[tid] = 0;
   const int64_t m0 = rowtile * TM;
   const E* src = (const E*)P.src;
   const int64_t nkt = (P.K + TK - 1) / TK;
+  auto take = [](unsigned& e, RowSpread& S, const E& v) {
+    if constexpr (SPREAD) {
+      if constexpr (CPLX) { spread_add(S, v.x); spread_add(S, v.y); }
+      else spread_add(S, v);
+    } else {
+      if constexpr (CPLX) e = max(e, max(exp_field(v.x), exp_field(v.y)));
+      else e = max(e, exp_field(v));
+    }
+  };
   if (!P.lanes_on_k) {
     // rows contiguous in the source: each thread keeps one row (tid % TM) and
     // walks k = tid / TM + j * (threads / TM) -- one offset, one maximum
@@ -1091,24 +1199,76 @@ __device__ __forceinline__ void rowmax_body(const GatherParams& P, int64_t rowti
     const int mm = tid % TM;
     const int64_t lm = m0 + mm < P.rows ? P.lm[m0 + mm] : -1;
     unsigned e = 0;
+    RowSpread S{0ull, 0u, 0u};
     if (lm >= 0) {
       for (int64_t kt = ky; kt < nkt; kt += kstep) {
         const int64_t k0 = kt * TK + tid / TM;
+        E v[TK / KS];  // all loads before the first is used
 #pragma unroll
         for (int it = 0; it < TK / KS; ++it) {
           const int64_t k = k0 + it * KS;
-          if (k < P.K) {
-            const E v = src[lm + P.lk[k]];
-            if constexpr (CPLX) e = max(e, max(exp_field(v.x), exp_field(v.y)));
-            else e = max(e, exp_field(v));
-          }
+          v[it] = k < P.K ? src[lm + P.lk[k]] : E{};
         }
+#pragma unroll
+        for (int it = 0; it < TK / KS; ++it) take(e, S, v[it]);
       }
     }
+    if constexpr (SPREAD) { e = S.e; sm_spread[tid] = S; }
     __syncthreads();
     if (e) atomicMax(&sm_max[mm], e);
     __syncthreads();
-    if (tid < TM && sm_max[tid] && m0 + tid < P.rows) atomicMax(&P.rowE[m0 + tid], sm_max[tid]);
+    if (tid < TM && m0 + tid < P.rows) {
+      if (sm_max[tid]) atomicMax(&P.rowE[m0 + tid], sm_max[tid]);
+      if constexpr (SPREAD) {
+#pragma unroll
+        for (int i = 1; i < KS; ++i) spread_merge(S, sm_spread[tid + i * TM]);
+        P.spread[(int64_t)ky * P.rows + m0 + tid] = S;
+      }
+    }
+    return;
+  }
+  if constexpr (SPREAD) {
+    // half a warp per row: a thread counts in TM / 16 rows only (16 rows a thread, as
+    // below, take 128 registers: 200 against 148 us for the 96/24 ladder)
+    constexpr int KL = 16, RR = TM * KL / kGThreads, KR = TK / KL;
+    const int kl = tid % KL, r0 = tid / KL;
+    int64_t lmv[RR];
+    RowSpread S[RR];
+#pragma unroll
+    for (int i = 0; i < RR; ++i) {
+      const int64_t m = m0 + r0 + i * (kGThreads / KL);
+      lmv[i] = m < P.rows ? P.lm[m] : -1;
+      S[i] = {0ull, 0u, 0u};
+    }
+    for (int64_t kt = ky; kt < nkt; kt += kstep) {
+      E v[RR][KR];  // all loads before the first is used
+#pragma unroll
+      for (int j = 0; j < KR; ++j) {
+        const int64_t k = kt * TK + kl + j * KL;
+        const int64_t lk = k < P.K ? P.lk[k] : 0;
+#pragma unroll
+        for (int i = 0; i < RR; ++i) v[i][j] = lmv[i] >= 0 && k < P.K ? src[lmv[i] + lk] : E{};
+      }
+#pragma unroll
+      for (int i = 0; i < RR; ++i)
+#pragma unroll
+        for (int j = 0; j < KR; ++j) {
+          if constexpr (CPLX) { spread_add(S[i], v[i][j].x); spread_add(S[i], v[i][j].y); }
+          else spread_add(S[i], v[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < RR; ++i) {
+      RowSpread T = S[i];
+#pragma unroll
+      for (int o = KL / 2; o > 0; o >>= 1)
+        spread_merge(T, RowSpread{__shfl_xor_sync(0xffffffffu, T.bins, o), __shfl_xor_sync(0xffffffffu, T.e, o), 0u});
+      const int64_t m = m0 + r0 + i * (kGThreads / KL);
+      if (kl == 0 && m < P.rows) {
+        if (T.e) atomicMax(&P.rowE[m], T.e);
+        P.spread[(int64_t)ky * P.rows + m] = T;
+      }
+    }
     return;
   }
   int64_t lmv[IT];
@@ -1147,13 +1307,13 @@ __device__ __forceinline__ void rowmax_body(const GatherParams& P, int64_t rowti
   if (tid < TM && sm_max[tid] && m0 + tid < P.rows) atomicMax(&P.rowE[m0 + tid], sm_max[tid]);
 }
 
-template <bool CPLX>
+template <bool CPLX, bool SPREAD>
 __global__ void __launch_bounds__(kGThreads) rowmax_kernel(const __grid_constant__ GatherPair Q) {
   const bool second = blockIdx.x >= Q.ctas_a;
   const unsigned x = second ? blockIdx.x - Q.ctas_a : blockIdx.x, rows = second ? Q.rows_b : Q.rows_a;
   const unsigned ky = x / rows, rt = x - ky * rows;
   const GatherParams P = second ? Q.b : Q.a;
-  rowmax_body<CPLX>(P, rt, (int)ky, second ? Q.gy_b : Q.gy_a);
+  rowmax_body<CPLX, SPREAD>(P, rt, (int)ky, second ? Q.gy_b : Q.gy_a);
 }
 
 template <bool CPLX>
@@ -1161,20 +1321,28 @@ __global__ void __launch_bounds__(kGThreads) rowmax_grouped_kernel(const GatherP
                                                                    const int2* __restrict__ map) {
   const int2 jm = map[blockIdx.x];
   const GatherParams P = jobs[jm.x];
-  rowmax_body<CPLX>(P, jm.y, blockIdx.y, gridDim.y);
+  rowmax_body<CPLX, false>(P, jm.y, blockIdx.y, gridDim.y);
 }
 
-// Grid of a launch over both operands: enough CTAs per operand to fill the GPU
-// several times over, each walking a strided set of K tiles.
+// CTAs per row tile of one operand: enough to fill the GPU several times over, each
+// walking a strided set of K tiles.
+int64_t k_splits(int64_t rows, int64_t kt) {
+  return std::max<int64_t>(1, std::min<int64_t>(kt, (int64_t)num_sms() * 16 / std::max<int64_t>(1, rows)));
+}
+template <bool CPLX>
+int rowmax_splits(int64_t rows, int64_t K) {
+  constexpr int64_t TM = CPLX ? gather_rows<double2>() : gather_rows<double>();
+  return (int)k_splits((rows + TM - 1) / TM, (K + kGK - 1) / kGK);
+}
+
+// Grid of a launch over both operands.
 int pair_grid(GatherPair* Q, const GatherParams& a, const GatherParams& b, int64_t rows_a, int64_t kt_a, int64_t rows_b,
               int64_t kt_b, unsigned* grid) {
-  auto gy = [](int64_t rows, int64_t kt) {
-    return std::max<int64_t>(1, std::min<int64_t>(kt, (int64_t)num_sms() * 16 / std::max<int64_t>(1, rows)));
-  };
-  const int64_t ga = gy(rows_a, kt_a), gb = gy(rows_b, kt_b);
+  const int64_t ga = k_splits(rows_a, kt_a), gb = k_splits(rows_b, kt_b);
   if (rows_a * ga + rows_b * gb > INT32_MAX) { set_error("gather grid too large"); return TB_ERR_LIMIT; }
   Q->a = a;
   Q->b = b;
+  Q->refused = nullptr;
   Q->rows_a = (unsigned)rows_a;
   Q->rows_b = (unsigned)rows_b;
   Q->gy_a = (int)ga;
@@ -1192,17 +1360,19 @@ int run_rowmax(const GatherParams& a, const GatherParams& b, cudaStream_t s) {
   if (int e = pair_grid(&Q, a, b, (a.rows + TM - 1) / TM, (a.K + kGK - 1) / kGK, (b.rows + TM - 1) / TM,
                         (b.K + kGK - 1) / kGK, &grid))
     return e;
-  rowmax_kernel<CPLX><<<grid, kGThreads, 0, s>>>(Q);
+  if (a.spread) rowmax_kernel<CPLX, true><<<grid, kGThreads, 0, s>>>(Q);
+  else rowmax_kernel<CPLX, false><<<grid, kGThreads, 0, s>>>(Q);
   TB_CHECK_LAUNCH();
   return 0;
 }
 
 template <int MODEA, int MODEB>
 int run_gather(const GatherParams& a, const GatherParams& b, int64_t rows_a, int64_t rows_b, int64_t ktiles,
-               cudaStream_t s) {
+               const unsigned* refused, cudaStream_t s) {
   GatherPair Q;
   unsigned grid;
   if (int e = pair_grid(&Q, a, b, rows_a, ktiles, rows_b, ktiles, &grid)) return e;
+  Q.refused = refused;
   constexpr int smem = std::max(gather_smem_bytes<MODEA>(), gather_smem_bytes<MODEB>());
   auto launch = [&](auto kern, DeviceOnce& once) -> int {
     const cudaError_t e = smem_limit_once(once, kern, smem);

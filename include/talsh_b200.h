@@ -50,7 +50,8 @@ typedef struct {
   int moduli;      /* R8/C8 fused: 0 (default) = modular residues (Ozaki scheme II) where the
                       contraction allows, with the fewest moduli that keep 46 bits per operand;
                       8..15 = that many moduli; -1 = INT8 slices (Ozaki scheme I) instead.
-                      A positive `slices` also selects INT8 slices. */
+                      A positive `slices` also selects INT8 slices.  The bits count from the
+                      largest value of an operand's row (column), not from each value. */
   int reserved[2];
 } tb_plan_t;
 
@@ -128,6 +129,12 @@ int tb_tensor_norm(int data_kind, size_t volume, const void* d, int which, doubl
  * shape comes back may, on its second call, time candidate plans with
  * alpha = 0, beta = 1 and wait for them (one host synchronisation per
  * shape; not while the stream is capturing) before running the fastest.
+ * R8 and C8 products that AUTO leaves to the plain method have the error bound
+ * of FP64 sums for every element, whatever the operands' magnitudes: where it
+ * multiplies them as residues (15 moduli), the GPU first counts how far the
+ * rows' values spread and runs FP64 sums instead where residues could be off
+ * by more.  What AUTO picks for the tensor cores is accurate relative to the
+ * rows' largest values.
  * Replaces gpu_tensor_block_contract_dlf
  * (TALSH/tensor_algebra_gpu_nvidia.cu:5847). */
 int tb_tensor_contract(const int* cptrn, int data_kind, int drank, const int* d_dims, void* d,
@@ -346,7 +353,8 @@ typedef struct {
                         terms); its tensor-core work is products * flops */
   int tile_n;        /* tensor-core N tile of the executed plan */
   int tile_m;        /* tensor-core M tile: 128 (one SM) or 256 (an SM pair, cta_group::2) */
-  int moduli;        /* R8/C8 fused with modular residues: moduli (one INT8 GEMM each); 0 otherwise */
+  int moduli;        /* R8/C8 fused with modular residues: moduli (one INT8 GEMM each); 0 otherwise.
+                        15 from AUTO: the GPU may have run FP64 sums instead (tb_tensor_contract) */
   int residue_bits;  /* ... and the bits p kept per operand (|X| <= 2^p) */
 } tb_contract_stats_t;
 int tb_last_contract_stats(tb_contract_stats_t* stats);

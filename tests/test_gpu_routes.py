@@ -52,6 +52,105 @@ def test_long_products_keep_51_bits(xt, dev, kind, dt, m, n, k, moduli):
     assert (torch.linalg.norm(out - want) / torch.linalg.norm(want)).item() <= 4e-15
 
 
+def install_plain():
+    """A caller's network that always picks the plain method."""
+    p = np.zeros(16 * 8 + 8 + 64 + 8 + 8 * XB.SELECT_PLANS + XB.SELECT_PLANS, np.float32)
+    p[-XB.SELECT_PLANS + 1:] = 9.0
+    XB.selector_install(8, p, np.zeros(16, np.float32), np.ones(16, np.float32))
+
+
+def spread_operands(kind, name, m, n, k, g):
+    """L as (m, k), R as (n, k) by the name of their magnitudes along k."""
+    real = lambda *s: torch.rand(*s, dtype=torch.float64, device="cuda", generator=g) * 2 - 1  # noqa: E731
+    mk = real if kind == XB.R8 else lambda *s: torch.complex(real(*s), real(*s))
+    l, r = mk(m, k), mk(n, k)
+    x = torch.arange(k, dtype=torch.float64, device="cuda")
+    if name == "graded":       # energy denominators: 1e-8 .. 1 along k in one operand, the inverse in the other
+        w = torch.pow(10.0, -8 * x / k)
+        l, r = l * w, r / w
+    elif name == "steep":      # 1 .. 2^-60
+        w = torch.pow(2.0, -torch.floor(60 * x / k))
+        l, r = l * w, r / w
+    elif name == "half":       # half of L tiny where R has values, R zero on the other half
+        l, r = l * torch.where(x < k // 2, 1.0, 1e-10), r * (x >= k // 2)
+    elif name == "lognormal":
+        l = l * torch.exp(3 * torch.randn(m, k, dtype=torch.float64, device="cuda", generator=g))
+        r = r * torch.exp(3 * torch.randn(n, k, dtype=torch.float64, device="cuda", generator=g))
+    elif name == "one row":
+        l[7] *= torch.pow(2.0, -torch.floor(60 * x / k))
+    elif name == "one column":
+        r[5] *= torch.pow(2.0, -torch.floor(60 * x / k))
+    elif name == "subnormal row":
+        l[3] *= 1e-310
+    elif name == "zero row and column":
+        l[3], r[n - 1] = 0, 0
+    elif name == "rows of all sizes":
+        l = l * torch.pow(10.0, torch.linspace(-150, 150, m, dtype=torch.float64, device="cuda"))[:, None]
+    return l.contiguous(), r.contiguous()
+
+
+@pytest.mark.parametrize("k_first", [True, False])
+@pytest.mark.parametrize("kind,m,n,k", [(XB.R8, 1400, 1100, 1290), (XB.C8, 900, 700, 1000), (XB.C8, 1300, 1200, 259)])
+@pytest.mark.parametrize("name,residues", [
+    ("uniform", True), ("zero row and column", True), ("rows of all sizes", True), ("graded", False), ("steep", False),
+    ("half", False), ("lognormal", False), ("one row", False), ("one column", False), ("subnormal row", False)])
+def test_fp64_products_keep_every_element(xt, dev, kind, m, n, k, k_first, name, residues):
+    """Whatever the magnitudes along k, every element of a product that the selector
+    leaves to the plain method is as close as an FP64 sum: within 2 sqrt(K) 2^-53
+    of sum |l| |r| (rounding errors of K random terms; the alternative, a fixed point
+    below a row's largest value, loses all digits of "steep").  Where the magnitudes
+    allow it the product runs as residues, else as the one-kernel form, bit for bit."""
+    g = torch.Generator(device="cuda").manual_seed(k + len(name))
+    l, r = spread_operands(kind, name, m, n, k, g)
+    pattern, ld, rd = ("D(i,j)+=L(k,i)*R(k,j)", [k, m], [k, n]) if k_first else ("D(i,j)+=L(i,k)*R(j,k)", [m, k], [n, k])
+    lt, rt = (l, r) if k_first else (l.T.contiguous(), r.T.contiguous())
+
+    def run():
+        d = torch.full((n, m), float("nan"), dtype=l.dtype, device="cuda")
+        xt.tensor_contract(pattern, kind, [m, n], d.data_ptr(), ld, lt.data_ptr(), rd, rt.data_ptr(), 1.0,
+                           accumulative=False, stream=torch.cuda.current_stream())
+        return d
+
+    XB.selector_install(0, None, None, None)  # the size rule, which leaves these products to the plain method
+    got, st = run(), xt.last_contract_stats()
+    assert st.moduli == 15 and st.residue_bits >= 51
+    install_plain()
+    try:
+        plain = run()
+        assert xt.last_contract_stats().moduli == 0
+    finally:
+        XB.selector_install(0, None, None, None)
+    assert torch.equal(got, plain) != residues
+    rows, cols = [0, 3, 7, 8, m // 2, m - 1], [0, 5, n // 2, n - 1]
+    wide = np.longdouble if kind == XB.R8 else np.clongdouble
+    lh, rh = l[rows].cpu().numpy().astype(wide), r[cols].cpu().numpy().astype(wide)
+    err = np.abs(got[cols][:, rows].cpu().numpy() - rh @ lh.T)
+    # (k 2^-1074: products that round among the subnormal numbers)
+    assert (err <= 2 * np.sqrt(k) * 2.0 ** -53 * (np.abs(rh) @ np.abs(lh).T) + k * 5e-324).all()
+
+
+def test_refused_residues_with_nan_and_accumulation(xt, dev):
+    """Falling magnitudes and a NaN row, D accumulated: the one-kernel form updates D once."""
+    m, n, k = 1400, 1100, 1290
+    g = torch.Generator(device="cuda").manual_seed(2)
+    l, r = spread_operands(XB.R8, "steep", m, n, k, g)
+    l[11, 4] = float("nan")
+    d0 = torch.rand(n, m, dtype=torch.float64, device="cuda", generator=g)
+    outs = []
+    XB.selector_install(0, None, None, None)
+    for network in (False, True):
+        if network:
+            install_plain()
+        try:
+            d = d0.clone()
+            xt.tensor_contract("D(i,j)+=L(k,i)*R(k,j)", XB.R8, [m, n], d.data_ptr(), [k, m], l.data_ptr(), [k, n],
+                               r.data_ptr(), -0.5, stream=torch.cuda.current_stream())
+        finally:
+            XB.selector_install(0, None, None, None)
+        outs.append(d)
+    assert torch.isnan(outs[0][:, 11]).all() and torch.equal(outs[0].nan_to_num(), outs[1].nan_to_num())
+
+
 @pytest.mark.parametrize("dtk,tol", [(O.R8, 1e-12), (O.C8, 1e-12), (O.R4, 1e-4), (O.C4, 1e-4)])
 @pytest.mark.parametrize("c", [3, 8, 19, 24])
 def test_blocked_rows(xt, dev, dtk, tol, c):
