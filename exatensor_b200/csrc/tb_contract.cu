@@ -372,34 +372,45 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
     //    us against 67 us).
     // A network of the caller's own keeps its choice of the tensor cores.  The
     // predictions are fits to measured times (about 5% and 15% off).
-    auto refine = [&](int picked, bool callers, int* err) {
-      const bool asked = plan && (plan->slices || plan->tile_n || plan->tile_m || plan->bf16_terms || plan->moduli);
-      if (picked == TB_METHOD_FUSED && (asked || callers)) return false;
-      // What the one-kernel form declines keeps the picked method: an output that
-      // overlaps an operand is multiplied from copies (TTGT), and for more groups
-      // than its parameter block holds nothing predicts the plain method's time.
-      DirectPlan dp;
-      if (direct_plan(Z, dtk, d, l, r, &dp) != 0) return false;
+    const bool asked = plan && (plan->slices || plan->tile_n || plan->tile_m || plan->bf16_terms || plan->moduli);
+    // What the one-kernel form declines keeps the picked method: an output that
+    // overlaps an operand is multiplied from copies (TTGT), and for more groups
+    // than its parameter block holds nothing predicts the plain method's time.
+    DirectPlan dp;
+    int direct = -1;
+    auto direct_ok = [&]() {
+      if (direct < 0) direct = direct_plan(Z, dtk, d, l, r, &dp) == 0;
+      return direct == 1;
+    };
+    // The plain method (see above) with the given alpha and accumulation; residues:
+    // whether 15 moduli may stand for it.
+    auto run_plain = [&](bool residues, double xr, double xi, int acc) -> int {
+      if (!direct_ok()) {
+        tb_plan_t tp{};
+        tp.method = TB_METHOD_TTGT;
+        return run_method(Z, dtk, ddims, d, ldims, l, rdims, r, xr, xi, acc, lconj, rconj, &tp, s);
+      }
       constexpr int64_t kExactMinK = 256;
-      if (picked == TB_METHOD_TTGT && is_double(dtk) && !callers && !asked && Z.K >= kExactMinK &&
-          predicted_fused_us(Z, dtk, 15) < dp.us) {
+      if (residues && is_double(dtk) && !asked && Z.K >= kExactMinK && predicted_fused_us(Z, dtk, 15) < dp.us) {
         tb_plan_t rp{};
         rp.method = TB_METHOD_FUSED;
         rp.moduli = 15;
-        const int fe = contract_fused(Z, dtk, ddims, d, ldims, l, rdims, r, ar, ai, accumulative != 0, lconj, rconj, &rp,
-                                      s, &g_stats, &dp);
+        const int fe = contract_fused(Z, dtk, ddims, d, ldims, l, rdims, r, xr, xi, acc != 0, lconj, rconj, &rp, s,
+                                      &g_stats, &dp);
         // short of scratch, or K too long for 51 bits: as before
         if (fe != TB_ERR_NO_MEMORY && fe != TB_ERR_NOT_IMPLEMENTED && fe != TB_ERR_LIMIT && fe != TB_ERR_INVALID_ARGS) {
           g_stats.method = TB_METHOD_FUSED;
-          *err = fe;
-          return true;
+          return fe;
         }
       }
-      if (picked == TB_METHOD_FUSED && dp.us >= predicted_fused_us(Z, dtk, 14)) return false;
       g_stats.method = TB_METHOD_TTGT;
       g_stats.gemm_launches = 1;
-      *err = run_direct(dp, dtk, cplx ? ar : real_alpha(ar, ai), cplx ? ai : 0.0, accumulative != 0, lconj, rconj, s);
-      return true;
+      return run_direct(dp, dtk, cplx ? xr : real_alpha(xr, xi), cplx ? xi : 0.0, acc != 0, lconj, rconj, s);
+    };
+    // Whether a product that was picked for the tensor cores, but not timed there, runs
+    // in one kernel instead.
+    auto small = [&](bool callers) {
+      return !asked && !callers && direct_ok() && dp.us < predicted_fused_us(Z, dtk, 14);
     };
     auto candidate = [&](int c) {
       tb_plan_t cp = plan ? *plan : tb_plan_t{};
@@ -409,7 +420,9 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
       if (c == kCandSlices) { cp.slices = 6; cp.moduli = -1; }
       return cp;
     };
-    if (selector_pick(f, &idx, &tune, &key) == 0) {
+    bool measured = false;  // idx was timed, now or on an earlier call: it stands
+    if (selector_pick(f, &idx, &tune, &key, &measured) == 0) {
+      const bool callers = selector_is_callers();
       if (tune) {
         // no timing (it waits on the host) while the stream is captured into a graph
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -425,6 +438,12 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
         // clock drift under the power cap does not favour the one timed first
         static const bool trace = [] { const char* e = getenv("TB_SELECT_TRACE"); return e && e[0] == '1'; }();
         constexpr int kRounds = 2;
+        // as it would run if picked: the plain method in the form that it takes
+        auto timed_run = [&](int c) {
+          if (c == 0) return run_plain(!callers, 0.0, 0.0, 1);
+          const tb_plan_t cp = candidate(c);
+          return run_method(Z, dtk, ddims, d, ldims, l, rdims, r, 0.0, 0.0, 1, lconj, rconj, &cp, s);
+        };
         float t[kNumCandidates];
         bool ok[kNumCandidates];
         cudaEvent_t e0, e1;
@@ -434,16 +453,14 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
           t[c] = 1e30f;
           ok[c] = false;
           if (!(tune & (1u << c))) continue;
-          tb_plan_t cp = candidate(c);
-          ok[c] = run_method(Z, dtk, ddims, d, ldims, l, rdims, r, 0.0, 0.0, 1, lconj, rconj, &cp, s) == 0;
+          ok[c] = timed_run(c) == 0;
           cudaGetLastError();
         }
         for (int round = 0; round < kRounds; ++round)
           for (int c = 0; c < kNumCandidates; ++c) {
             if (!ok[c]) continue;
-            tb_plan_t cp = candidate(c);
             cudaEventRecord(e0, s);
-            const int ce = run_method(Z, dtk, ddims, d, ldims, l, rdims, r, 0.0, 0.0, 1, lconj, rconj, &cp, s);
+            const int ce = timed_run(c);
             cudaEventRecord(e1, s);
             float ms = 0.f;
             if (!ce && cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess)
@@ -464,17 +481,18 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         selector_remember(key, idx);
+        measured = true;
         std::memset(&g_stats, 0, sizeof(g_stats));
         g_stats.m = Z.M; g_stats.n = Z.N; g_stats.k = Z.K;
         g_stats.flops = (cplx ? 8.0 : 2.0) * (double)Z.M * (double)Z.N * (double)Z.K;
       }
-      if (refine(idx == 0 ? TB_METHOD_TTGT : TB_METHOD_FUSED, selector_is_callers(), &e)) return e;
+      if (idx == 0 || (!measured && small(callers))) return run_plain(idx == 0 && !callers, ar, ai, accumulative);
       learned = candidate(idx);
       return run_method(Z, dtk, ddims, d, ldims, l, rdims, r, ar, ai, accumulative, lconj, rconj, &learned, s,
                         /*fallback=*/true);
     }
     method = select_method(dtk, Z, plan);
-    if (refine(method, false, &e)) return e;
+    if (method == TB_METHOD_TTGT || small(false)) return run_plain(method == TB_METHOD_TTGT, ar, ai, accumulative);
   }
   if (method == TB_METHOD_AUTO) method = TB_METHOD_TTGT;
   learned = plan ? *plan : tb_plan_t{};

@@ -41,8 +41,9 @@ constexpr int kCandPair = 3;
 constexpr int kCandSlices = 4;
 constexpr int kNumCandidates = 5;
 // The network's choice for a descriptor (idx), or the cached measured one;
-// tune_mask: candidates to time before choosing (0: none).
-int selector_pick(const float* features, int* idx, unsigned* tune_mask, uint64_t* key);
+// tune_mask: candidates to time before choosing (0: none); measured: the choice was
+// timed on an earlier call.
+int selector_pick(const float* features, int* idx, unsigned* tune_mask, uint64_t* key, bool* measured);
 void selector_remember(uint64_t key, int idx);
 // Whether the caller installed the network in use: its choice of the tensor
 // cores then stands, where the library would refine its own network's.

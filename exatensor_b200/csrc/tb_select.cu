@@ -142,7 +142,8 @@ int best_plan(const float* f, const float* y) {
   return best;
 }
 
-int selector_pick(const float* f, int* idx, unsigned* tune_mask, uint64_t* key) {
+int selector_pick(const float* f, int* idx, unsigned* tune_mask, uint64_t* key, bool* measured) {
+  *measured = false;
   Selector& S = sel();
   std::lock_guard<std::mutex> lk(S.mu);
   if (!S.on) return -1;
@@ -172,6 +173,7 @@ int selector_pick(const float* f, int* idx, unsigned* tune_mask, uint64_t* key) 
     auto it = S.cache.find(h);
     if (it != S.cache.end()) {
       *idx = it->second;
+      *measured = true;
       mask = 0;
     } else {
       if (S.seen.size() >= kMaxRemembered) S.seen.clear();

@@ -9,6 +9,10 @@ uniform data) and the FP64 reference itself carries about sqrt(K) 2^-54.
 The fused path's rows run in blocks of eight of the left operand's contiguous
 group when D's fastest group is another one: groups shorter than a block, whole
 blocks, and blocks with a remainder."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -19,6 +23,7 @@ from tests.test_gpu_contract import oracle_dd
 from tests.test_gpu_permute import rand_host
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 @pytest.mark.parametrize("kind,dt,m,n,k,moduli", [(XB.R8, torch.float64, 1400, 1100, 1290, 15),
@@ -149,6 +154,38 @@ def test_refused_residues_with_nan_and_accumulation(xt, dev):
             XB.selector_install(0, None, None, None)
         outs.append(d)
     assert torch.isnan(outs[0][:, 11]).all() and torch.equal(outs[0].nan_to_num(), outs[1].nan_to_num())
+
+
+MEASURED = """
+import torch
+import exatensor_b200 as XB
+XB.device_init(0)
+a, b, c, d = 395, 470, 294, 417
+l, r = torch.rand(d * c * a, device="cuda"), torch.rand(c * b * d, device="cuda")
+out = torch.zeros(b * a, device="cuda")
+for _ in range(3):
+    XB.tensor_contract("D(a,b)+=L(a,c,d)*R(d,b,c)", XB.R4, [a, b], out.data_ptr(), [a, c, d], l.data_ptr(), [d, b, c],
+                       r.data_ptr(), 1.0, accumulative=False, stream=torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    st = XB.last_contract_stats()
+print("ran", st.method, st.tile_n, st.tile_m)
+"""
+
+
+def test_a_measured_choice_runs():
+    """What timing the candidates chose (on the second call of a large shape, by the
+    shipped network) is what runs, then and later."""
+    env = dict(os.environ, TB_SELECT_TRACE="1")
+    r = subprocess.run([sys.executable, "-c", MEASURED], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    line = [x for x in r.stderr.splitlines() if x.startswith("tb_select:")]
+    assert line, "the candidates were timed"
+    pick = int(line[-1].split("->")[1])
+    ran = [int(x) for x in r.stdout.split("ran")[1].split()]
+    if pick == 0:
+        assert ran[0] == XB.METHOD_TTGT
+    else:
+        assert ran == [XB.METHOD_FUSED, 128 if pick == 1 else 256, 256 if pick == 3 else 128]
 
 
 @pytest.mark.parametrize("dtk,tol", [(O.R8, 1e-12), (O.C8, 1e-12), (O.R4, 1e-4), (O.C4, 1e-4)])
