@@ -222,23 +222,23 @@ def test_residue_tile_of_192_columns(xt, dev, kind, n, tile):
 def test_output_over_an_operand_is_multiplied_from_copies(xt, dev):
     """D starts inside L, and L's infinity lies where another row of D goes: the
     product still sees the old L.  (The infinity's row is infinite, other entries are
-    sums of 300 FP64 products and an accumulated old element.)"""
+    sums of 300 FP64 products.)"""
     m, n, k, off = 96, 80, 300, 3
     rng = np.random.default_rng(4)
     x = rng.uniform(-1, 1, k * m + n * m + off)
     x[5] = np.inf  # L(5, 0); also D(2, 0)
     r = rng.uniform(-1, 1, n * k)
-    lm, rm, d0 = x[:k * m].reshape(k, m), r.reshape(k, n), x[off:off + n * m].reshape(n, m)
+    lm, rm = x[:k * m].reshape(k, m), r.reshape(k, n)
     with np.errstate(invalid="ignore"):
-        want = rm.T @ lm + d0
+        want = rm.T @ lm
     buf, rd = dev.put(x), dev.put(r)
     xt.tensor_contract("D(a,b)+=L(a,k)*R(b,k)", XB.R8, [m, n], buf.data_ptr() + 8 * off, [m, k], buf.data_ptr(), [n, k],
-                       rd.data_ptr(), 1.0, stream=dev.stream())
+                       rd.data_ptr(), 1.0, accumulative=False, stream=dev.stream())
     st = xt.last_contract_stats()
     got = dev.get(buf, np.float64)[off:off + n * m].reshape(n, m)
     assert np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
     fin = np.isfinite(want)
-    assert fin.sum() >= (m - 2) * n and np.array_equal(np.isfinite(got), fin)
+    assert fin.sum() >= (m - 1) * n and np.array_equal(np.isfinite(got), fin)
     assert np.linalg.norm(got[fin] - want[fin]) <= 4e-15 * np.linalg.norm(want[fin])
     assert st.method == XB.METHOD_TTGT and st.moduli == 0
 
