@@ -19,21 +19,21 @@ template <typename E, int WM, int WN, int KW, int MI, int NI, int BK, int ST, in
 struct Variant {
   using S = Shape<E, WM, WN, KW, MI, NI, BK, ST>;
   static TileShape shape() { return {S::BM, S::BN, S::BKT, S::T, OCC}; }
-  static int launch(const Params& P, int64_t ctas, cudaStream_t s) {
+  static int launch(const Params& P, int64_t ctas, cudaStream_t s, const unsigned* when) {
     if constexpr (!Elem<E>::F32) {  // conditional launches: FP64 data only
-      if (P.when) return launch_as<true>(P, ctas, s);
+      if (when) return launch_as(P, ctas, s, when);
     }
-    return launch_as<false>(P, ctas, s);
+    return launch_as(P, ctas, s);
   }
-  template <bool WHEN>
-  static int launch_as(const Params& P, int64_t ctas, cudaStream_t s) {
+  template <class... Word>
+  static int launch_as(const Params& P, int64_t ctas, cudaStream_t s, Word... when) {
     static DeviceOnce attr;
-    auto kern = direct_kernel<E, WM, WN, KW, MI, NI, BK, ST, OCC, WHEN>;
+    auto kern = direct_kernel<E, WM, WN, KW, MI, NI, BK, ST, OCC, Word...>;
     const size_t smem = S::smem(P.split > 1 || KW > 1);
     cudaError_t e = smem_limit_once(attr, kern, (int)S::smem(true));
     if (e != cudaSuccess) { set_error("direct contraction smem attribute: %s", cudaGetErrorString(e)); return TB_ERR_CUDA; }
     if (P.split == 1) {
-      kern<<<(unsigned)ctas, S::T, smem, s>>>(P);
+      kern<<<(unsigned)ctas, S::T, smem, s>>>(P, when...);
     } else {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3((unsigned)ctas, 1, 1);
@@ -46,7 +46,7 @@ struct Variant {
       a.val.clusterDim.y = a.val.clusterDim.z = 1;
       cfg.attrs = &a;
       cfg.numAttrs = 1;
-      e = cudaLaunchKernelEx(&cfg, kern, P);
+      e = cudaLaunchKernelEx(&cfg, kern, P, when...);
       if (e != cudaSuccess) {
         cudaGetLastError();
         set_error("direct contraction cluster launch: %s", cudaGetErrorString(e));
@@ -60,7 +60,7 @@ struct Variant {
 
 struct VariantRef {
   TileShape sh;
-  int (*launch)(const Params&, int64_t, cudaStream_t);
+  int (*launch)(const Params&, int64_t, cudaStream_t, const unsigned*);
 };
 template <class V>
 VariantRef ref() { return {V::shape(), &V::launch}; }
@@ -119,7 +119,6 @@ int direct_plan(const Matricization& Z, int dtk, const void* d, const void* l, c
 int run_direct(const DirectPlan& plan, int dtk, double ar, double ai, bool accumulate, int lconj, int rconj,
                cudaStream_t s, const unsigned* when) {
   Params P = plan.P;
-  P.when = when;
   P.ar = ar;
   P.ai = ai;
   P.br = accumulate ? 1.0 : 0.0;
@@ -127,7 +126,7 @@ int run_direct(const DirectPlan& plan, int dtk, double ar, double ai, bool accum
   P.aconj = plan.swap ? rconj : lconj;
   P.bconj = plan.swap ? lconj : rconj;
   const int ts = timed_begin(s);
-  const int e = variants(dtk)[plan.variant].launch(P, plan.ctas, s);
+  const int e = variants(dtk)[plan.variant].launch(P, plan.ctas, s, when);
   timed_end(ts, s);
   return e;
 }

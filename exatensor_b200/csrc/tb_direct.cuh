@@ -98,17 +98,18 @@ __device__ __forceinline__ void update(const Params& P, bool read_d, E* d, const
   *d = w;
 }
 
-// WHEN: does nothing unless the word P.when is set (a kernel of its own, since waiting
-// for one parameter before all others costs every launch 0.4 us).
-template <typename E, int WM, int WN, int KW, int MI, int NI, int BK, int ST, int OCC, bool WHEN>
-__global__ void __launch_bounds__(WM* WN* KW * 32, OCC) direct_kernel(const __grid_constant__ Params P) {
+// Word: nothing, or the address of a word without which set the kernel does nothing (a
+// kernel of its own, since waiting for one parameter before all others costs every
+// launch 0.4 us).
+template <typename E, int WM, int WN, int KW, int MI, int NI, int BK, int ST, int OCC, class... Word>
+__global__ void __launch_bounds__(WM* WN* KW * 32, OCC) direct_kernel(const __grid_constant__ Params P, Word... when) {
   using S = Shape<E, WM, WN, KW, MI, NI, BK, ST>;
   using R = typename Elem<E>::R;
   using Acc = typename Elem<E>::Acc;
   constexpr bool CPLX = Elem<E>::CPLX;
   constexpr int BM = S::BM, BN = S::BN, BKT = S::BKT, T = S::T, NC = CPLX ? 2 : 1;
-  if constexpr (WHEN) {
-    if (!*P.when) return;
+  if constexpr (sizeof...(Word) > 0) {
+    if ((!*when || ...)) return;
   }
   extern __shared__ __align__(16) unsigned char direct_smem[];
   int64_t* row_a = reinterpret_cast<int64_t*>(direct_smem);

@@ -39,7 +39,6 @@ struct Side {
 };
 
 struct Params {
-  const unsigned* when;      // set: the launch does nothing unless this word is
   const void* A;
   const void* B;
   void* D;
