@@ -102,6 +102,11 @@ constexpr double kL2PerUs = 8.4e6;
 constexpr double kFixedUs = 7.5;           // launch, offset tables and write-out of one round of CTAs
 constexpr double kRoundUs = 3.0;           // each further round
 constexpr double kKTileUs = 1.05;          // latency of one K tile
+// CTAs per SM that fit, by data kind (R4, R8, C4, C8) and shape; and CTAs resident at
+// once in clusters of 2, 4 and 8, at one to five per SM: a cluster stays within a GPC,
+// so that the larger ones leave SMs empty (cudaOccupancyMaxActiveClusters on B200).
+constexpr int kFit[4][7] = {{3, 3, 3, 3, 2, 5, 4}, {3, 3, 3, 3, 2, 3, 2}, {4, 3, 3, 3, 1, 1, 0}, {3, 3, 2, 2, 1, 1, 0}};
+constexpr int kResident[3][5] = {{148, 296, 444, 592, 740}, {132, 284, 416, 568, 700}, {120, 264, 384, 568, 688}};
 }  // namespace
 
 int plan_direct(const Matricization& Z, int es, bool cplx, const void* d, const void* l, const void* r,
@@ -199,9 +204,17 @@ int plan_direct(const Matricization& Z, int es, bool cplx, const void* d, const 
         const double eff = cplx ? kEffCplx[v] : kEffReal[v];
         const double fma = per_sm * sh.bm * sh.bn * kk * (cplx ? 4 : 1) / (kFmaPerUs * eff);
         const double lat = std::ceil(per_sm / sh.occ) * (kRoundUs + kKTileUs * kt);
+        // clusters that do not fit wait for a whole round of the others and then run
+        // nearly alone: 416 CTAs in clusters of 8 took 1.5 times their work's time
+        double stretch = 1.0;
+        if (split > 1) {
+          const int fit = kFit[(cplx ? 2 : 0) + (es == (cplx ? 16 : 8) ? 1 : 0)][v], lg = split == 2 ? 0 : split == 4 ? 1 : 2;
+          const double full = ctas / kResident[lg][fit - 1] * 148.0 / sms, part = full - std::floor(full);
+          if (full > 1.0) stretch = (std::floor(full) + (part > 0.0 ? std::max(0.5, part) : 0.0)) / full;
+        }
         const double hbm = (dbytes + abytes + bbytes) / kHbmPerUs;
         const double l2 = (abytes * amp * nt + bbytes * (b_seq ? 1.0 : sector) * mt + dbytes) / kL2PerUs;
-        const double us = kFixedUs + std::sqrt(fma * fma + lat * lat + hbm * hbm + l2 * l2) + 0.5 * (split - 1);
+        const double us = kFixedUs + std::sqrt(stretch * stretch * (fma * fma + lat * lat) + hbm * hbm + l2 * l2) + 0.5 * (split - 1);
         if (us < out->us) {
           out->us = us;
           out->variant = (int)v;

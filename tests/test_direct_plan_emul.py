@@ -41,6 +41,42 @@ def test_shapes_match_the_kernels():
     assert got == want
 
 
+@pytest.fixture(scope="module")
+def info(tmp_path_factory):
+    return build_info(tmp_path_factory)
+
+
+def build_info(tmp_path_factory):
+    """plans(cases): (variant, split, box, a_on_k, b_on_k, predicted us) per (pattern, extents, es, cplx), None where declined."""
+    exe = str(tmp_path_factory.mktemp("direct_info") / "direct_plan_info")
+    subprocess.run(["g++", "-O2", "-std=c++17", os.path.join(HERE, "emul", "direct_plan_info.cpp"),
+                    os.path.join(CSRC, "tb_direct_plan.cpp"), os.path.join(CSRC, "tb_pattern.cpp"), "-o", exe],
+                   check=True)
+
+    def plans(cases):
+        lines = []
+        for pat, ext, es, cplx in cases:
+            g = labels(pat)
+            flat = [len(x) for x in g] + [ext[c] for x in g for c in x] + list(O.parse_pattern(pat)[0]) + [es, int(cplx)]
+            lines.append(" ".join(map(str, flat)))
+        out = subprocess.run([exe], input="\n".join(lines), capture_output=True, text=True, check=True).stdout.splitlines()
+        assert len(out) == len(cases)
+        return [None if x == "DECLINED" else tuple(float(y) for y in x.split()) for x in out]
+
+    return plans
+
+
+def test_clusters_that_do_not_fit_at_once_are_predicted_slower(info):
+    """416 CTAs in clusters of eight, of which 384 are resident: measured 3.9 ms (R4, 395
+    x 470 x 122598).  The model has to stay within a third of that, or products that the
+    tensor cores run in 2.0 ms come here; a shape of which five CTAs per SM fit does
+    not wait (2183 x 33 x 24640, measured 0.40 ms)."""
+    long_sum, fits = info([("D(a,b)+=L(a,c,d)*R(d,b,c)", dict(a=395, b=470, c=294, d=417), 4, False),
+                           ("D(a,b,c)+=L(a,d,e,c)*R(e,b,d)", dict(a=37, b=33, c=59, d=140, e=176), 4, False)])
+    assert long_sum[5] > 3950 / 1.33
+    assert fits[5] < 400 * 1.33
+
+
 def test_every_index_once(emul):
     rng = random.Random(5)
     lines = []
