@@ -414,6 +414,46 @@ bool build_elem_plan(int es, int rank, const int* dims, const int* cptrn, int64_
   return true;
 }
 
+// What the element kernel cannot do fast is to read a line of the input per element:
+// it moves 1.5 (4-byte copies) to 2.6 TB/s then, where a warp that shares lines moves
+// 2.5 to 5.  The tiled engine is ahead of that where its plan moves whole vectors in
+// short, even tiles, from the sizes below on; with odd extents it is not (0.7 to 2
+// TB/s).  And where elements that share a sector are far apart in the output, sectors
+// of a large tensor leave L2 before their next use (16^6 R8 additions of 128 MB: 321 us
+// against 77).  Over 1900 random and regular permutations of both kernels on B200 this
+// rule is within 8% of the element kernel where it turns from it, and twice to four
+// times as fast at best.
+bool tiled_is_ahead(const ElemPermParams& E, int es, bool add, int rank, const int* dims, const int* cptrn, int in_align) {
+  const double mb = (double)E.vol * es / 1048576.0;
+  if (mb < (add ? (es == 4 ? 7.5 : es == 8 ? 28.0 : 80.0) : es == 4 ? 7.0 : es == 8 ? 14.0 : 1e9)) return false;
+  // the first 32 outputs of a row share no 128-byte line of the input
+  double before = 1.0, near = 1.0, reach = 0.0;  // near: inputs in a row within 1024 outputs; reach: outputs between them
+  for (int d = 0; d < E.rank; ++d) {
+    if (before < 32.0 && E.ext[d] > 1 && (double)E.sin[d] * es < 128.0) return false;
+    if (E.sin[d] == 1) {
+      reach = before;
+      near = std::min((double)E.ext[d], std::max(1.0, 1024.0 / before));
+    }
+    before *= E.ext[d];
+  }
+  PermParams P;
+  if (build_perm_plan_o2n(es, rank, dims, cptrn, &P)) return false;
+  const int la = P.LA * es, lb = P.LB * es;
+  const bool even = la <= 2048 && lb >= 256;
+  const bool lists = even && (P.rows2d ? perm2d_list_entries(P, true, 256) : P.vec2d ? perm2d_list_entries(P, false, 256) : 0) > 0;
+  bool whole = true;
+  for (int i = 0; i < P.rank; ++i) whole = whole && P.dims[i] % P.tile[i] == 0;
+  const bool vec = even && !lists && whole && perm_glist_vector_bytes(P, in_align, 256) == 16;
+  if (!add) {
+    if (es == 4) return (lists && near < 16.0) || (near < 2.0 && ((P.lin2d && even) || (vec && mb >= 12.0)));
+    return near < 2.0 && (lists || (vec && mb >= 18.0));
+  }
+  if (es == 4) return (lists && whole && near < 16.0 && P.ntiles >= 500) || (vec && near < 2.0 && P.ntiles >= 800 && mb >= 14.0);
+  if (near >= 2.0 || !whole) return false;
+  if (mb >= 80.0 && reach * 32.0 >= (es == 8 ? 7.0 : 17.0) * 1048576.0) return true;
+  return lists && P.ntiles >= 800 && mb >= (es == 8 ? 28.0 : 100.0);
+}
+
 int perm_glist_vector_bytes(const PermParams& P, int in_align, int nthr) {
   const int es = P.es;
   int vb = es;

@@ -140,6 +140,9 @@ TB_HD void elem_digit(const ElemPermParams& P, int d, uint32_t* rest, uint32_t* 
 // (and 2^31 - 2^20 elements, kElemRank dims after merging).  False otherwise, and
 // for a pattern that is no permutation (the general path reports it).
 bool build_elem_plan(int es, int rank, const int* dims, const int* cptrn, int64_t max_bytes, ElemPermParams* P);
+// Whether the tiled engine is ahead of the element kernel on a permutation below the
+// latter's size limits (add: permuted addition; in_align: of the input pointer).
+bool tiled_is_ahead(const ElemPermParams& E, int es, bool add, int rank, const int* dims, const int* cptrn, int in_align);
 
 // Bytes of one pipeline stage (a tile in shared memory).
 inline int64_t perm_stage_bytes(const PermParams& P) { return (int64_t)P.nA * P.lap * P.es; }

@@ -123,9 +123,9 @@ int run_scatter(int rank, const int* dims, const int* cptrn, const E* in, const 
   return 0;
 }
 
-// Bytes of a tensor up to which the element kernel runs: where, over random
-// permutations of ranks 2 to 6 with inputs that change from call to call, it stops
-// being ahead of the tiled engine.  Mean us, tiled against element: copies of
+// Bytes of a tensor up to which the element kernel runs (where tiled_is_ahead does not
+// say otherwise): where, over random permutations of ranks 2 to 6 with inputs that
+// change from call to call, it stops being ahead of the tiled engine on average.  Mean us, tiled against element: copies of
 // 4-byte elements 29.0 / 26.5 at 24 MB and 25.9 / 28.3 at 32 MB, of 8-byte ones 23.0
 // / 19.1 at 32 MB, of 16-byte ones 17.5 / 15.5 at 32 MB; additions 84.6 / 66.2 at 64
 // MB and 206 / 232 at 128 MB, 88 / 81 at 128 MB and 183 / 211 at 260 MB, 175 / 121 at
@@ -141,6 +141,15 @@ constexpr int64_t elem_limit(int es, bool rmw) {
 bool elem_allowed() {
   static const bool on = !getenv("TB_PERM_LOADS");
   return on;
+}
+
+// Plans the element kernel where it is the choice for a permutation.
+template <typename E, typename Store>
+bool elem_is_choice(int rank, const int* dims, const int* cptrn, const E* in, ElemPermParams* S) {
+  constexpr bool add = is_rmw_store<Store>::value;
+  const uintptr_t a = (uintptr_t)in;
+  return elem_allowed() && build_elem_plan((int)sizeof(E), rank, dims, cptrn, elem_limit(sizeof(E), add), S) &&
+         !tiled_is_ahead(*S, (int)sizeof(E), add, rank, dims, cptrn, a % 16 == 0 ? 16 : a % 8 == 0 ? 8 : (int)sizeof(E));
 }
 
 template <typename E, typename Store>
@@ -271,10 +280,7 @@ int run_copy_measured(int rank, const int* dims, const int* cptrn, const E* in, 
   // (tuning and test switch; results are identical)
   static const int tma_env = [] { const char* e = getenv("TB_PERM_TMA"); return e ? (e[0] == '1' ? 1 : 0) : -1; }();
   ElemPermParams S;
-  if (tma_env != 1 && elem_allowed()) {
-    if (build_elem_plan((int)sizeof(E), rank, dims, cptrn, elem_limit(sizeof(E), is_rmw_store<Store>::value), &S))
-      return launch_elem<E, Store>(S, in, st, s);
-  }
+  if (tma_env != 1 && elem_is_choice<E, Store>(rank, dims, cptrn, in, &S)) return launch_elem<E, Store>(S, in, st, s);
   int64_t vol = 1;
   for (int i = 0; i < rank; ++i) vol *= dims[i];
   std::vector<int> key{(int)sizeof(E), rank};
@@ -368,9 +374,7 @@ int run_copy_measured(int rank, const int* dims, const int* cptrn, const E* in, 
   return 0;
 }
 
-// Runs a permutation with the tiled engine, or the scatter kernel when the
-// plan builder declines the layout.
-// Runs a permutation with the tiled engine, or the scatter kernel when the
+// Runs a permutation with the element kernel, the tiled engine, or the scatter kernel when the
 // plan builder declines the layout.  Used where output must be written once
 // (the fused add), so nothing is timed: the plan is the one the measured
 // choice keeps for copies of the same shape and element size when there is
@@ -382,9 +386,7 @@ int run_permutation(int rank, const int* dims, const int* cptrn, const E* in, co
                     cudaStream_t s, bool force_scatter = false) {
   if (!force_scatter) {
     ElemPermParams S;
-    if (elem_allowed() &&
-        build_elem_plan((int)sizeof(E), rank, dims, cptrn, elem_limit(sizeof(E), is_rmw_store<Store>::value), &S))
-      return launch_elem<E, Store>(S, in, st, s);
+    if (elem_is_choice<E, Store>(rank, dims, cptrn, in, &S)) return launch_elem<E, Store>(S, in, st, s);
     std::vector<int> key{(int)sizeof(E), rank};
     key.insert(key.end(), dims, dims + rank);
     key.insert(key.end(), cptrn, cptrn + rank);
