@@ -15,6 +15,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <numeric>
 #include <unordered_map>
 #include <vector>
@@ -51,14 +52,39 @@ struct OpBlock {          // one distinct operand block in the A (row) or B (col
   size_t plane_off;               // bytes into the plane buffer
 };
 
-// Plan memory from the device's pool, which keeps what earlier plans gave back
-// (cudaMalloc maps fresh memory each time: 2 ms for a few hundred MB).  Plans are
-// created on one stream and used on others: creation ends with a synchronization,
-// and a plan's memory goes back only after the device is idle.
+// Plan memory, from a pool of its own on every device that keeps up to kPlanPoolKeep
+// bytes of what closed plans gave back, three times the 3.6 GB of the 4-segment ladder,
+// whose creation takes 9 ms with and 41 ms without them, and returns the rest to the
+// device.  Plans are created on one
+// stream and used on others: creation ends with a synchronization, and a plan's
+// memory goes back only after the device is idle.
+constexpr uint64_t kPlanPoolKeep = (uint64_t)12 << 30;
+
+cudaMemPool_t plan_pool(int dev) {
+  static std::mutex mu;
+  static cudaMemPool_t pools[64] = {};
+  std::lock_guard<std::mutex> lk(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    uint64_t keep = kPlanPoolKeep;
+    if (cudaMemPoolCreate(&pools[dev], &props) != cudaSuccess) {
+      cudaGetLastError();
+      pools[dev] = nullptr;
+    } else {
+      cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+  }
+  return pools[dev];
+}
+
 void* dalloc(size_t bytes, int* err, cudaStream_t s) {
   void* p = nullptr;
   if (*err) return nullptr;
-  if (cudaMallocAsync(&p, std::max<size_t>(bytes, 256), s) != cudaSuccess) {
+  cudaMemPool_t pool = plan_pool(current_device());
+  if (!pool || cudaMallocFromPoolAsync(&p, std::max<size_t>(bytes, 256), pool, s) != cudaSuccess) {
     cudaGetLastError();
     set_error("block-sparse plan: device allocation of %zu bytes failed", bytes);
     *err = TB_ERR_NO_MEMORY;
@@ -72,6 +98,7 @@ void* dalloc(size_t bytes, int* err, cudaStream_t s) {
 
 struct tb_bsc_plan_s {
   int dtk = 0;
+  int dev = 0;                     // the device it was made on
   bool i8 = true;
   bool resid = false;              // FP64 by modular residues (else INT8 slices)
   tb::ResiduePlan rp;              // residues: moduli and reconstruction constants
@@ -319,11 +346,26 @@ int set_slices(tb_bsc_plan_s* pl, int S, cudaStream_t s) {
 
 namespace {
 
-void plan_free(tb_bsc_plan_s* pl) {
-  drop_graph(pl);
-  if (!pl->allocs.empty()) cudaDeviceSynchronize();
-  for (void* p : pl->allocs) cudaFreeAsync(p, 0);
+// Frees a plan on its own device, whichever is current, once that device is idle.
+int plan_free(tb_bsc_plan_s* pl) {
+  const int cur = current_device();
+  cudaError_t e = cur != pl->dev ? cudaSetDevice(pl->dev) : cudaSuccess;
+  if (e == cudaSuccess) {
+    drop_graph(pl);
+    if (!pl->allocs.empty()) {
+      e = cudaDeviceSynchronize();
+      for (void* p : pl->allocs)
+        if (const cudaError_t f = cudaFreeAsync(p, 0); e == cudaSuccess) e = f;
+      // idle again: the pool lets go of what it holds above its limit
+      if (const cudaError_t f = cudaStreamSynchronize(0); e == cudaSuccess) e = f;
+    }
+    if (cur != pl->dev) cudaSetDevice(cur);
+  }
   delete pl;
+  if (e == cudaSuccess) return 0;
+  cudaGetLastError();
+  set_error("block-sparse plan: freeing its memory: %s", cudaGetErrorString(e));
+  return TB_ERR_CUDA;
 }
 
 template <typename T>
@@ -365,6 +407,7 @@ int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t*
     if (PP.cptrn[i] == 1) swap = false;
   auto* pl = new tb_bsc_plan_s();
   pl->dtk = dtk;
+  pl->dev = current_device();
   pl->i8 = dtk == kR8;
   {
     // attribute set here, before any graph capture of the plan's launches
@@ -824,8 +867,5 @@ extern "C" int tb_bsc_plan_info(const tb_bsc_plan_t* pl, tb_bsc_info_t* info) {
 }
 
 extern "C" int tb_bsc_plan_destroy(tb_bsc_plan_t* pl) {
-  if (!pl) return 0;
-  cudaDeviceSynchronize();
-  plan_free(pl);
-  return 0;
+  return pl ? plan_free(pl) : 0;
 }

@@ -174,3 +174,27 @@ def test_wide_blocks_and_long_block_sums(xt, dev, dtk, tol, tile_n):
         dt = O.NP_DTYPE[dtk]
         assert O.rel_frobenius(values(D, D.data, dt), values(D, ref, dt)) <= tol, (i, tile_n)
         plan.close()
+
+
+def matrix_task(d, l, r, m, n, k):
+    """D(a,i) += L(a,c) R(c,i) as one block task."""
+    return (d.data_ptr(), [m, n], l.data_ptr(), [m, k], r.data_ptr(), [k, n])
+
+
+def test_closed_plans_give_their_memory_back(xt, dev):
+    """Of a closed plan's 16 GB of planes at most the pool's 12 GB stay with the library."""
+    import torch
+    m, n, k = 50000, 256, 25000
+    l, r, d = [torch.empty(x, dtype=torch.float64, device="cuda") for x in (m * k, k * n, m * n)]
+    for t in (l, r, d):
+        t.uniform_(-1, 1)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    plan = XB.BlockSparsePlan("D(a,i)+=L(a,c)*R(c,i)", O.R8, [matrix_task(d, l, r, m, n, k)], accumulative=False,
+                              stream=dev.stream())
+    plan.execute(stream=dev.stream())
+    torch.cuda.synchronize()
+    held = before - torch.cuda.mem_get_info()[0]
+    plan.close()
+    assert held > 16 << 30
+    assert before - torch.cuda.mem_get_info()[0] <= (12 << 30) + (64 << 20)
