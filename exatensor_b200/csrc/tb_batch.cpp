@@ -21,11 +21,13 @@
 #include <vector>
 
 #include "talsh_b200.h"
+#include "tb_bsc.h"
 #include "tb_pattern.h"
 
 namespace {
 
 constexpr size_t kMaxCachedPlans = 8;
+constexpr size_t kMaxCachedBytes = (size_t)24 << 30;  // of all cached plans' planes together, as one plan may hold
 constexpr int kR4 = 4, kR8 = 8;  // TAL-SH data kinds the grouped kernel takes
 
 struct CachedPlan {
@@ -81,6 +83,18 @@ extern "C" int tb_batch_pending(const tb_batch_t* b) { return b ? (int)b->queue.
 
 namespace {
 
+// Closes the least recently used plans until at most `plans` are left, with at most
+// kMaxCachedBytes of planes unless it is one.
+void trim_cache(tb_batch_t* b, size_t plans) {
+  size_t bytes = 0;
+  for (auto& c : b->cache) bytes += tb::bsc_plan_bytes(c.plan);
+  while (b->cache.size() > plans || (b->cache.size() > 1 && bytes > kMaxCachedBytes)) {
+    bytes -= tb::bsc_plan_bytes(b->cache.back().plan);
+    tb_bsc_plan_destroy(b->cache.back().plan);
+    b->cache.pop_back();
+  }
+}
+
 int run_loop(tb_batch_t* b, void* stream) {
   tb::ParsedPattern P;
   tb::parse_pattern(b->pattern.c_str(), &P);
@@ -114,18 +128,22 @@ extern "C" int tb_batch_flush(tb_batch_t* b, void* stream) {
       b->stats.plan_reuses++;
     } else {
       tb_bsc_plan_t* pl = nullptr;
-      err = tb_bsc_plan_create(b->pattern.c_str(), b->dtk, (int)b->queue.size(), b->queue.data(), b->ar, b->ai,
-                               b->accumulative, b->has_plan ? &b->plan : nullptr, &pl, stream);
+      auto create = [&] {
+        return tb_bsc_plan_create(b->pattern.c_str(), b->dtk, (int)b->queue.size(), b->queue.data(), b->ar, b->ai,
+                                  b->accumulative, b->has_plan ? &b->plan : nullptr, &pl, stream);
+      };
+      err = create();
+      if (err == TB_ERR_NO_MEMORY && !b->cache.empty()) {  // without the cached plans
+        trim_cache(b, 0);
+        err = create();
+      }
       if (err == TB_ERR_NOT_IMPLEMENTED) {
         pl = nullptr;
         err = run_loop(b, stream);  // a pattern the grouped kernel does not take
       } else if (!err) {
         b->stats.plans_built++;
-        if (b->cache.size() >= kMaxCachedPlans) {
-          tb_bsc_plan_destroy(b->cache.back().plan);
-          b->cache.pop_back();
-        }
         b->cache.push_front(CachedPlan{std::move(key), pl, 0});
+        trim_cache(b, kMaxCachedPlans);
       }
       if (!pl) {
         if (!err) b->stats.tasks += (int64_t)b->queue.size();

@@ -20,6 +20,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "tb_bsc.h"
 #include "tb_bsc_gemm.cuh"
 #include "tb_tc_prep.cuh"
 
@@ -99,6 +100,7 @@ void* dalloc(size_t bytes, int* err, cudaStream_t s) {
 struct tb_bsc_plan_s {
   int dtk = 0;
   int dev = 0;                     // the device it was made on
+  size_t plane_bytes = 0;          // operand and residue planes
   bool i8 = true;
   bool resid = false;              // FP64 by modular residues (else INT8 slices)
   tb::ResiduePlan rp;              // residues: moduli and reconstruction constants
@@ -567,6 +569,7 @@ int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t*
   int err = 0;
   pl->tables = upload(pl, tab, &err, s);
   pl->planes = (unsigned char*)dalloc(plane_bytes, &err, s);
+  pl->plane_bytes = plane_bytes;
   if (pl->planes) pl->allocs.push_back(pl->planes);
   pl->n_erows = erows;
   pl->rowE = (unsigned*)dalloc(erows * sizeof(unsigned), &err, s);
@@ -648,6 +651,7 @@ int plan_create(const char* pattern, int dtk, int ntasks, const tb_block_task_t*
       bytes += (size_t)pl->rp.rs.n * rup(Ds[d].M, 128) * rup(Ds[d].N, 256);
     }
     res = (uint8_t*)dalloc(bytes, &err, s);
+    pl->plane_bytes += bytes;
     if (res) pl->allocs.push_back(res);
     if (err) { plan_free(pl); return err; }
   }
@@ -772,6 +776,8 @@ int build_graph(tb_bsc_plan_s* pl) {
 }
 
 }  // namespace
+
+size_t tb::bsc_plan_bytes(const tb_bsc_plan_t* plan) { return plan->plane_bytes; }
 
 extern "C" int tb_bsc_plan_create(const char* pattern, int data_kind, int ntasks, const tb_block_task_t* tasks,
                                   double alpha_real, double alpha_imag, int accumulative, const tb_plan_t* plan,

@@ -267,7 +267,8 @@ int tb_bsc_tasks_from_blocks(const char* pattern, const tb_block_list_t* d, cons
  * flushed before (same tasks, same order) reuses its plan and CUDA graph; on
  * its second use the plan's tile and slice choice is timed once.  The
  * accumulative flag applies to each output block once per flush.  Blocks
- * must stay allocated while a cached plan may run them. */
+ * must stay allocated while a cached plan may run them; the cached plans of a
+ * batch hold at most 24 GB of planes together (or one plan). */
 typedef struct tb_batch_s tb_batch_t;
 typedef struct {
   long long tasks;         /* tasks flushed */

@@ -91,3 +91,28 @@ def test_batch_rejects_bad_requests(xt):
         XB.Batch("D(a)+=L(a)", O.R8)      # not a contraction
     with pytest.raises(XB.TBError):
         XB.Batch(PATTERN, 3)              # not a data kind
+
+
+def test_cached_plans_are_bounded_together(xt, dev):
+    """Six lists whose plans hold 5.3 GB of planes each: at most four (24 GB) stay cached,
+    and a list whose plan was closed is planned again and gives the same result."""
+    import torch
+    from tests.test_gpu_bsc import matrix_task
+    m, n, k = 20000, 64, 20000
+    l = torch.empty(m * k, dtype=torch.float64, device="cuda").uniform_(-1, 1)
+    r = torch.empty(k * n, dtype=torch.float64, device="cuda").uniform_(-1, 1)
+    ds = [torch.empty(m * n, dtype=torch.float64, device="cuda") for _ in range(6)]
+    torch.cuda.synchronize()
+    b = XB.Batch("D(a,i)+=L(a,c)*R(c,i)", O.R8, accumulative=False)
+    for d in ds + ds[:1]:
+        d.zero_()
+        b.add([matrix_task(d, l, r, m, n, k)])
+        b.flush(stream=dev.stream())
+    torch.cuda.synchronize()
+    st = b.stats()
+    assert st.cached_plans == 4 and st.plans_built == 7 and st.plan_reuses == 0
+    assert all(torch.equal(d, ds[1]) for d in ds)
+    want = (r.view(n, k)[:, :].unsqueeze(0) @ l.view(k, m)[:, :50]).squeeze(0)  # the first 50 rows
+    got = ds[0].view(n, m)[:, :50]
+    assert torch.linalg.norm(got - want) <= 1e-12 * torch.linalg.norm(want)
+    b.close()
