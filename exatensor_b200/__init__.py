@@ -336,6 +336,10 @@ class BlockSparsePlan:
         _check(lib().tb_bsc_plan_info(self._h, C.byref(inf)))
         return inf
 
+    def moduli(self) -> int:
+        """Moduli of a plan that runs as modular residues, else 0."""
+        return lib().tb_bsc_plan_moduli(self._h)
+
     def close(self):
         if self._h:
             lib().tb_bsc_plan_destroy(self._h)

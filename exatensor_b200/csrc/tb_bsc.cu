@@ -4,9 +4,9 @@
 // under one index pattern, where several tasks may add into the same output
 // block (ExaTENSOR's TAVP-WRK issues them one talsh_tensor_contract per block,
 // INTERVIRT/tavp_worker.F90:9420-9518, call at :9467).  The plan built here
-// converts every distinct operand block once (row maxima, then INT8 slices or
-// BF16 parts, through per-block offset tables: two grouped launches over all
-// blocks) and runs all (output tile, pair) work in one persistent grouped GEMM
+// converts every distinct operand block once (row maxima, then residues, INT8
+// slices or BF16 parts, through per-block offset tables: two grouped launches over
+// all blocks) and runs all (output tile, pair) work in one persistent grouped GEMM
 // (tb_bsc_gemm.cuh) fed from a device-side queue.  The launch sequence is
 // captured once in a CUDA graph and replayed.  An autotuner times the tile
 // width and slice-count candidates on the plan's own data and keeps the
@@ -871,6 +871,8 @@ extern "C" int tb_bsc_plan_info(const tb_bsc_plan_t* pl, tb_bsc_info_t* info) {
     for (int s = 0; s < 2; ++s) info->tune_ms[b * 2 + s] = pl->tune_ms[b][s];
   return 0;
 }
+
+extern "C" int tb_bsc_plan_moduli(const tb_bsc_plan_t* pl) { return !pl ? -1 : pl->resid ? pl->rp.rs.n : 0; }
 
 extern "C" int tb_bsc_plan_destroy(tb_bsc_plan_t* pl) {
   return pl ? plan_free(pl) : 0;

@@ -184,7 +184,8 @@ int tb_tensor_contract_noalloc(const int* cptrn, int data_kind, int drank, const
  * same output block.  ExaTENSOR's TAVP-WRK runs such lists as one
  * talsh_tensor_contract per block (INTERVIRT/tavp_worker.F90:9420-9518, call
  * at :9467); these calls run the whole list as one grouped tensor-core
- * launch (R8: INT8 slices, R4: split BF16), replayed from a CUDA graph. */
+ * launch (R8: modular residues or INT8 slices, R4: split BF16), replayed from a
+ * CUDA graph. */
 typedef struct {
   void* d;           /* output block body (device, dlf) */
   const void* l;     /* left operand block body */
@@ -198,17 +199,22 @@ typedef struct tb_bsc_plan_s tb_bsc_plan_t;
 
 typedef struct {
   int tasks, left_blocks, right_blocks, out_blocks, work_items;
-  int slices;        /* INT8 slices (R8) */
+  int slices;        /* INT8 slices (R8) of a plan that runs slices (tb_bsc_plan_moduli) */
   int tile_n;        /* GEMM N tile */
   double flops;      /* sum of 2*M*N*K over the tasks */
-  float tune_ms[4];  /* autotuner timings: (tile 128, 6 slices), (128, 7), (256, 6), (256, 7) */
+  float tune_ms[4];  /* autotuner timings: (tile 128, 6 slices), (128, 7), (256, 6), (256, 7);
+                        without slices the second and fourth are 0 */
 } tb_bsc_info_t;
 
 /* Builds the plan: distinct operand blocks, offset tables, tensor maps and the
  * work list (device memory owned by the plan; blocks must stay allocated).
  * beta = accumulative ? 1 : 0 applies to every output block once per execution.
- * plan may set slices (R8, 2..7, default 6; planes are allocated for
- * max(slices, 6)) and tile_n (128 or 256). */
+ * R8 runs as modular residues, 14 or so exact INT8 products with 46 bits per
+ * operand below its row's largest value, unless plan asks for slices (slices =
+ * 2..7, or moduli = -1 for 6 of them; planes are allocated for max(slices, 6)),
+ * an output block sums more than 130944 contracted values, the planes would take
+ * more than 24 GB, or they cannot be allocated; other values of moduli leave
+ * their number to the library.  plan may set tile_n (128 or 256) too. */
 int tb_bsc_plan_create(const char* pattern, int data_kind, int ntasks, const tb_block_task_t* tasks,
                        double alpha_real, double alpha_imag, int accumulative, const tb_plan_t* plan,
                        tb_bsc_plan_t** out, void* stream);
@@ -217,11 +223,14 @@ int tb_bsc_plan_create(const char* pattern, int data_kind, int ntasks, const tb_
 int tb_bsc_execute(tb_bsc_plan_t* plan, void* stream);
 /* The same launches queued directly on the stream (no graph). */
 int tb_bsc_execute_stream(tb_bsc_plan_t* plan, void* stream);
-/* Times the tile-width candidates (and 6 vs 7 slices when the planes hold 7)
+/* Times the tile-width candidates (and 6 vs 7 slices when slice planes hold 7)
  * on the plan's data, with alpha = 0 and beta = 1 so that D is unchanged, and
  * keeps the fastest. */
 int tb_bsc_autotune(tb_bsc_plan_t* plan, void* stream);
 int tb_bsc_plan_info(const tb_bsc_plan_t* plan, tb_bsc_info_t* info);
+/* The moduli of a plan that runs as modular residues, 0 of one that runs INT8
+ * slices or split BF16 (-1 for a null plan). */
+int tb_bsc_plan_moduli(const tb_bsc_plan_t* plan);
 int tb_bsc_plan_destroy(tb_bsc_plan_t* plan);
 
 /* Diagnostic of the calling thread's last talshTensorContractXL: the D

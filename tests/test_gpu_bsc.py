@@ -198,3 +198,62 @@ def test_closed_plans_give_their_memory_back(xt, dev):
     plan.close()
     assert held > 16 << 30
     assert before - torch.cuda.mem_get_info()[0] <= (12 << 30) + (64 << 20)
+
+
+ARITHMETIC = [("residues", {}), ("slices", dict(moduli=-1)), ("slices", dict(slices=7))]
+
+
+def plan_of(xt, dev, tasks, arithmetic, options, **kw):
+    plan = XB.BlockSparsePlan(PATTERN, O.R8, tasks, plan=xt.make_plan(**options), stream=dev.stream(), **kw)
+    assert (plan.moduli() > 0) == (arithmetic == "residues")
+    return plan
+
+
+@pytest.mark.parametrize("arithmetic,options", ARITHMETIC)
+def test_each_arithmetic_replays_tunes_and_matches(xt, dev, arithmetic, options):
+    """Grouped result, graph replay, launches without the graph, and tuning, by residues
+    and by slices (six, and seven so that the tuner times both), against the
+    per-block loop."""
+    import torch
+    L, R, D, tasks, _ = make_problem(xt, dev, O.R8, seed=23)
+    d0 = D.data.clone()
+    ref = per_block_loop(xt, dev, O.R8, D, tasks, -0.75, True)
+    plan = plan_of(xt, dev, tasks, arithmetic, options, alpha=-0.75)
+    outs = []
+    for graph in (True, True, False):
+        D.data.copy_(d0)
+        plan.execute(stream=dev.stream(), graph=graph)
+        torch.cuda.synchronize()
+        outs.append(D.data.clone())
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    assert O.rel_frobenius(values(D, outs[0], np.float64), values(D, ref, np.float64)) <= 1e-12
+    D.data.copy_(d0)
+    plan.autotune(stream=dev.stream())
+    torch.cuda.synchronize()
+    assert torch.equal(D.data, d0)
+    inf = plan.info()
+    timed = [x > 0 for x in inf.tune_ms]
+    assert timed == ([True] * 4 if options.get("slices") == 7 else [True, False, True, False])
+    assert arithmetic == "residues" or inf.slices in (6, 7)
+    plan.execute(stream=dev.stream())
+    torch.cuda.synchronize()
+    xt.device_check(dev.stream())
+    assert O.rel_frobenius(values(D, D.data, np.float64), values(D, ref, np.float64)) <= 1e-12
+    plan.close()
+
+
+@pytest.mark.parametrize("arithmetic,options", ARITHMETIC[:2])
+@pytest.mark.parametrize("tile_n", [128, 256])
+def test_each_arithmetic_on_wide_blocks(xt, dev, arithmetic, options, tile_n):
+    """256 x 3072 output blocks, and blocks whose rows and columns end inside tiles."""
+    import torch
+    for segl, segr in [([[16], [16], [8], [8, 16]], [[8], [8, 16], [64], [48]]),
+                       ([[13, 5], [11], [7], [9]], [[7], [9], [17], [3, 31]])]:
+        L, R, D, tasks = fixed_problem(xt, dev, O.R8, segl, segr, 60)
+        ref = per_block_loop(xt, dev, O.R8, D, tasks, 1.0, False)
+        plan = plan_of(xt, dev, tasks, arithmetic, dict(options, tile_n=tile_n), accumulative=False)
+        plan.execute(stream=dev.stream())
+        torch.cuda.synchronize()
+        xt.device_check(dev.stream())
+        assert O.rel_frobenius(values(D, D.data, np.float64), values(D, ref, np.float64)) <= 1e-12
+        plan.close()
