@@ -224,7 +224,10 @@ __device__ __forceinline__ void epilogue_pass(const EP& P, uint32_t tcol, bool m
         const int ce = __shfl_sync(0xffffffffu, ce_l, j);
         if (!mval || n0 + j >= P.N || ((skipc >> j) & 1u)) continue;
         T v;
-        if (OZ) v = (T)(P.ar * scale2((double)(int)r[j], re + ce - shift));
+        // grouped products have no fix-up: rows and columns with a NaN or an infinity become NaN
+        if (OZ && !std::is_same<EP, TcGemmParams>::value && (re >= kNonFiniteExp || ce >= kNonFiniteExp))
+          v = (T)__longlong_as_double(0x7FF8000000000000ll);
+        else if (OZ) v = (T)(P.ar * scale2((double)(int)r[j], re + ce - shift));
         else v = (T)P.ar * __uint_as_float(r[j]);
         T o;
         if (!first) o = old[j] + v;

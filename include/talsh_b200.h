@@ -214,7 +214,8 @@ typedef struct {
  * 2..7, or moduli = -1 for 6 of them; planes are allocated for max(slices, 6)),
  * an output block sums more than 130944 contracted values, the planes would take
  * more than 24 GB, or they cannot be allocated; other values of moduli leave
- * their number to the library.  plan may set tile_n (128 or 256) too. */
+ * their number to the library.  plan may set tile_n (128 or 256) too.  An output row
+ * (column) whose operand row holds a NaN or an infinity becomes NaN. */
 int tb_bsc_plan_create(const char* pattern, int data_kind, int ntasks, const tb_block_task_t* tasks,
                        double alpha_real, double alpha_imag, int accumulative, const tb_plan_t* plan,
                        tb_bsc_plan_t** out, void* stream);

@@ -257,3 +257,33 @@ def test_each_arithmetic_on_wide_blocks(xt, dev, arithmetic, options, tile_n):
         xt.device_check(dev.stream())
         assert O.rel_frobenius(values(D, D.data, np.float64), values(D, ref, np.float64)) <= 1e-12
         plan.close()
+
+
+@pytest.mark.parametrize("arithmetic,options", ARITHMETIC[:2])
+def test_nan_and_infinity_in_a_block(xt, dev, arithmetic, options):
+    """Rows and columns of the output whose operand rows hold a NaN or an infinity are NaN
+    throughout; all others are what they are without them."""
+    import torch
+    segl, segr = [[13], [11], [7], [9]], [[7], [9], [17], [3, 31]]
+    L, R, D, tasks = fixed_problem(xt, dev, O.R8, segl, segr, 70)
+    plan = plan_of(xt, dev, tasks, arithmetic, options, accumulative=False)
+    plan.execute(stream=dev.stream())
+    clean = {k: D.data.view(torch.float64)[o:o + int(np.prod(d))].clone() for k, (o, d) in D.blocks.items()}
+    lv, rv = L.data.view(torch.float64), R.data.view(torch.float64)
+    off = L.blocks[(0, 0, 0, 0)][0]
+    lv[off + 5 + 13 * 2 + 13 * 11 * 3] = float("nan")       # a = 5, b = 2
+    lv[off + 7 + 13 * 10 + 13 * 11 * 20] = float("inf")     # a = 7, b = 10
+    off = R.blocks[(0, 0, 0, 1)][0]
+    rv[off + 4 + 63 * 8 + 63 * 17 * 30] = float("-inf")     # i = 8, j = 30 of the second block
+    plan.execute(stream=dev.stream())
+    torch.cuda.synchronize()
+    for key, (o, dims) in D.blocks.items():
+        got = D.data.view(torch.float64)[o:o + int(np.prod(dims))].view(tuple(reversed(dims)))  # j, i, b, a
+        want = clean[key].view(tuple(reversed(dims))).clone()
+        want[:, :, 2, 5] = float("nan")
+        want[:, :, 10, 7] = float("nan")
+        if key[3] == 1:
+            want[30, 8] = float("nan")
+        assert torch.equal(torch.isnan(got), torch.isnan(want)), key
+        assert torch.equal(got.nan_to_num(), want.nan_to_num()), key
+    plan.close()
