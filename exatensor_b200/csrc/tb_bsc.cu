@@ -17,6 +17,7 @@
 #include <cstring>
 #include <mutex>
 #include <numeric>
+#include <string>
 #include <unordered_map>
 #include <vector>
 
@@ -786,11 +787,14 @@ extern "C" int tb_bsc_plan_create(const char* pattern, int data_kind, int ntasks
   if (!device_error_word()) { set_error("tb_bsc_plan_create: device error word unavailable"); return TB_ERR_CUDA; }
   if (int e = bsc_prepare_attrs()) return e;
   tb_bsc_plan_s* pl = nullptr;
+  const std::string before = tb_last_error();
   int e = plan_create(pattern, data_kind, ntasks, tasks, alpha_real, alpha_imag, accumulative, plan, &pl,
                       (cudaStream_t)stream, true);
-  if (e == TB_ERR_NO_MEMORY)  // without the residue planes
+  if (e == TB_ERR_NO_MEMORY) {  // without the residue planes
+    set_error("%s", before.c_str());
     e = plan_create(pattern, data_kind, ntasks, tasks, alpha_real, alpha_imag, accumulative, plan, &pl,
                     (cudaStream_t)stream, false);
+  }
   if (e) return e;
   *out = pl;
   return 0;

@@ -26,6 +26,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <string>
 #include <mutex>
 #include <vector>
 
@@ -395,6 +396,7 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
         tb_plan_t rp{};
         rp.method = TB_METHOD_FUSED;
         rp.moduli = 15;
+        const std::string before = tb_last_error();
         const int fe = contract_fused(Z, dtk, ddims, d, ldims, l, rdims, r, xr, xi, acc != 0, lconj, rconj, &rp, s,
                                       &g_stats, &dp);
         // short of scratch, or K too long for 51 bits: as before
@@ -402,6 +404,7 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
           g_stats.method = TB_METHOD_FUSED;
           return fe;
         }
+        set_error("%s", before.c_str());  // not this call's failure
       }
       g_stats.method = TB_METHOD_TTGT;
       g_stats.gemm_launches = 1;

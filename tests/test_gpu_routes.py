@@ -262,3 +262,39 @@ def test_more_groups_than_the_one_kernel_form_holds(xt, dev):
     axis = {perm[rank - 1 - i]: i + 1 for i in range(rank)}
     want = c.transpose([0] + [axis[rank - 1 - i] for i in range(rank)]).ravel()
     assert np.linalg.norm(dev.get(dd, np.float64) - want) <= 4e-15 * np.linalg.norm(want)
+
+
+def test_short_of_scratch_the_one_kernel_form_runs(xt, dev):
+    """With no memory for the residue planes (0.1 GB here) a long FP64 product runs in one
+    kernel, and the call that succeeded leaves no error text."""
+    from cuda.bindings import driver as cu
+    m, n, k = 1400, 1100, 1290
+    g = torch.Generator(device="cuda").manual_seed(1)
+    l, r = [torch.rand(x, k, dtype=torch.float64, device="cuda", generator=g) - 0.5 for x in (m, n)]
+    d = torch.zeros(n, m, dtype=torch.float64, device="cuda")
+
+    def run():
+        xt.tensor_contract("D(i,j)+=L(k,i)*R(k,j)", XB.R8, [m, n], d.data_ptr(), [k, m], l.data_ptr(), [k, n],
+                           r.data_ptr(), 1.0, accumulative=False, stream=torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        return xt.last_contract_stats()
+
+    install_plain()  # (both forms run once, so that their kernels are loaded before memory runs short)
+    run()
+    XB.selector_install(0, None, None, None)
+    assert run().moduli == 15
+    want = r @ l.T
+    d.zero_()
+    text = xt.lib().tb_last_error()
+    err, pool = cu.cuDeviceGetDefaultMemPool(torch.cuda.current_device())
+    assert cu.cuMemPoolTrimTo(pool, 0)[0] == cu.CUresult.CUDA_SUCCESS
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        st = run()
+        assert xt.lib().tb_last_error() == text
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert st.method == XB.METHOD_TTGT and st.moduli == 0
+    assert torch.linalg.norm(d - want) <= 4e-15 * torch.linalg.norm(want)
