@@ -66,6 +66,21 @@ def build_info(tmp_path_factory):
     return plans
 
 
+def test_device_cases_cover_the_shapes(info):
+    """The planner takes the tile shape, split and box for which each case of the device
+    test (tests/test_gpu_direct_shapes.py) is listed; together they hold every shape that
+    it takes for products of up to 1e9 multiply-adds."""
+    import json
+    cases = json.load(open(os.path.join(HERE, "golden", "direct_cases.json")))
+    es = {"R4": 4, "R8": 8, "C4": 8, "C8": 16}
+    got = info([(c[4], {x.split("=")[0]: int(x.split("=")[1]) for x in c[5].split()}, es[c[0]], c[0][0] == "C") for c in cases])
+    assert [c[:4] for c in cases] == [[c[0], int(p[0]), int(p[1]), int(p[2])] for c, p in zip(cases, got)]
+    for kind, shapes in (("R4", 7), ("R8", 7), ("C4", 5), ("C8", 5)):
+        mine = [c for c in cases if c[0] == kind]
+        assert {c[1] for c in mine} == set(range(shapes))
+        assert {c[2] for c in mine} == {1, 2, 4, 8} and {c[3] for c in mine} == {0, 1}
+
+
 def test_clusters_that_do_not_fit_at_once_are_predicted_slower(info):
     """416 CTAs in clusters of eight, of which 384 are resident: measured 3.9 ms (R4, 395
     x 470 x 122598).  The model has to stay within a third of that, or products that the
