@@ -136,10 +136,13 @@ constexpr int64_t elem_limit(int es, bool rmw) {
              : (es == 4 ? (int64_t)24 << 20 : ((int64_t)32 << 20) - 1);
 }
 
-// TB_PERM_LOADS (a tuning knob) names a load mechanism of the tiled engine: no
-// element kernel then.
+// No element kernel where TB_PERM_LOADS (a tuning knob) names a load mechanism of the
+// tiled engine, or with TB_PERM_ELEM=0 (tuning and test switch; results are identical).
 bool elem_allowed() {
-  static const bool on = !getenv("TB_PERM_LOADS");
+  static const bool on = [] {
+    const char* e = getenv("TB_PERM_ELEM");
+    return !getenv("TB_PERM_LOADS") && !(e && e[0] == '0');
+  }();
   return on;
 }
 

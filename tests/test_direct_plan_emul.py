@@ -75,7 +75,7 @@ def test_device_cases_cover_the_shapes(info):
     es = {"R4": 4, "R8": 8, "C4": 8, "C8": 16}
     got = info([(c[4], {x.split("=")[0]: int(x.split("=")[1]) for x in c[5].split()}, es[c[0]], c[0][0] == "C") for c in cases])
     assert [c[:4] for c in cases] == [[c[0], int(p[0]), int(p[1]), int(p[2])] for c, p in zip(cases, got)]
-    for kind, shapes in (("R4", 7), ("R8", 7), ("C4", 5), ("C8", 5)):
+    for kind, shapes in (("R4", 7), ("R8", 7), ("C4", 5), ("C8", 6)):
         mine = [c for c in cases if c[0] == kind]
         assert {c[1] for c in mine} == set(range(shapes))
         assert {c[2] for c in mine} == {1, 2, 4, 8} and {c[3] for c in mine} == {0, 1}
