@@ -9,7 +9,7 @@
 // contracted indices itself, gathers the operand tiles with cp.async straight
 // into the multiplication's shared-memory layout, and writes D through its
 // offsets.  What bounds it: D's traffic for short contracted indices, FP64
-// tensor throughput (mma.sync m8n8k4, the only FP64 tensor instruction) for
+// tensor throughput (by mma.sync m8n8k4; the larger FP64 shapes are not tried) for
 // long ones, and the launch for small ones.  Measured, us, TTGT / this: 121 x 25 x
 // 121 R8 54 / 12; 324 x 325 x 104 R8 49 / 13; 6859 x 6859 x 19 R8 (752 MB of D traffic)
 // 520 / 239; R4 index transform 373248 x 24 x 72 245 / 117.  Staging every product in
@@ -23,27 +23,12 @@
 
 #include <type_traits>
 
+#include "tb_async.cuh"
 #include "tb_common.cuh"
 #include "tb_direct_plan.h"
 
 namespace tb {
 namespace direct {
-
-template <int BYTES>
-__device__ __forceinline__ void gather_async(void* sdst, const void* gsrc, bool valid) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(sdst);
-  const int n = valid ? BYTES : 0;
-  if constexpr (BYTES == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gsrc), "r"(n) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(gsrc), "n"(BYTES), "r"(n) : "memory");
-}
-
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
 
 template <typename E>
 struct Elem {
@@ -177,7 +162,7 @@ __global__ void __launch_bounds__(WM* WN* KW * 32, OCC) direct_kernel(const __gr
         for (int it = 0; it < IT; ++it) {
           const int64_t ro = row[r0 + it * (T / BKT)];
           const bool ok = (ro | kf) >= 0;
-          gather_async<(int)sizeof(E)>(d + it * (T / BKT) * pitch, base + (ok ? ro : 0), ok);
+          cp_async_elem<(int)sizeof(E)>(d + it * (T / BKT) * pitch, base + (ok ? ro : 0), ok);
         }
       } else {
         int r = tid % ROWS, pos = r;
@@ -197,7 +182,7 @@ __global__ void __launch_bounds__(WM* WN* KW * 32, OCC) direct_kernel(const __gr
           if (kk >= kend) break;
           const int64_t kf = kof[kk];
           const bool ok = (ro | kf) >= 0;
-          gather_async<(int)sizeof(E)>(d + it * (T / ROWS) * pitch, base + (ok ? kf : 0), ok);
+          cp_async_elem<(int)sizeof(E)>(d + it * (T / ROWS) * pitch, base + (ok ? kf : 0), ok);
         }
       }
     };

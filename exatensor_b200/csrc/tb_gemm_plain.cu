@@ -5,6 +5,7 @@
 //   R8: FP64 tensor-core MMA (mma.sync m8n8k4 f64; tcgen05 has no FP64 kind)
 //   C8: the same MMA on real/imaginary fragments (4 real products)
 //   R4, C4: FP32 FFMA on the CUDA cores
+#include "tb_async.cuh"
 #include "tb_common.cuh"
 #include "tb_gemm.h"
 
@@ -30,12 +31,6 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src, bool pred)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
-
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
-}
 
 // ------------------------------------------------------------------ R8 -----
 constexpr int D_BM = 128, D_BN = 128, D_BK = 16, D_LD = 20, D_ST = 3;

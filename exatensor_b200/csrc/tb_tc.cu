@@ -139,7 +139,8 @@ int select_method(int dtk, const Matricization& Z, const tb_plan_t* plan) {
 // whole rounds of work units (10^6 operations), output bytes (MB) and rounds,
 // weighted by a fit to 212 random contractions on B200 (5% rms for R8, 8% for
 // R4): a round of units costs its MMAs plus about 3 us, D's bytes run at 2.6 to
-// 4.4 TB/s, operands at 4 to 7 TB/s.
+// 4.4 TB/s, operands at 4 to 7 TB/s.  Products that take 192-wide tiles are predicted
+// as by 256-wide ones: three tiles of 192 columns took 7% less than three of 256.
 double predicted_fused_us(const Matricization& Z, int dtk, int n) {
   const bool cplx = is_complex(dtk), f64 = is_double(dtk);
   bool swap = false;  // rows: the operand holding D's fastest dimension
@@ -219,11 +220,11 @@ int contract_fused(const Matricization& Z0, int dtk, const int* ddims, void* d, 
   const int64_t K = Z.K;
   const int64_t Kr = cplx ? 2 * K : K, Nr = cplx ? 2 * Nc : Nc;
   const int64_t Kpad = round_up(Kr, 128);
-  // N tile: what the plan asks for, else 256 (128 for narrow products).  The residue
-  // GEMM is bound by the bytes that its tiles read from L2 (128 + BN rows of 128 bytes
-  // per K block), so without a request it takes 192 where that reads a twelfth less:
-  // N = 576 in three tiles of 192 instead of three of 256 (9216 x 576 x 9216 by 15
-  // moduli: 1589 -> 1553 us in all).
+  // N tile: what the plan asks for, else 256 (128 for narrow products).  Without a
+  // request residue products take 192 where the tiles then read a twelfth less (128 +
+  // BN rows of 128 bytes per K block), which is where fewer of their columns are
+  // padding: N = 576 in three tiles of 192 instead of three of 256 (9216 x 576 x 9216
+  // by 15 moduli: GEMM 642 -> 597 us, 1589 -> 1553 us in all).
   const bool asks_tile = plan && (plan->tile_n == 128 || plan->tile_n == 256);
   int BN = asks_tile ? plan->tile_n : Nr >= 192 ? 256 : 128;
   if (!asks_tile && i8 && !(plan && (plan->slices > 0 || plan->moduli < 0 || plan->tile_m == 256)) && Nr > 128 &&

@@ -13,6 +13,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "tb_async.cuh"
 #include "tb_common.cuh"
 #include "tb_pattern.h"
 #include "tb_tc_gemm.cuh"
@@ -414,18 +415,6 @@ template <int MODE>
 constexpr int gather_smem_bytes() {
   using T = GatherTile<MODE>;
   return 2 * T::BUF + 3 * T::TK * 8 + T::TM * 20;
-}
-
-// Asynchronous copy of one element into shared memory; zero-filled when
-// !valid (src is then any valid address and is not read).
-template <int BYTES>
-__device__ __forceinline__ void cp_async_elem(void* sdst, const void* gsrc, bool valid) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(sdst);
-  const int n = valid ? BYTES : 0;
-  if constexpr (BYTES == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gsrc), "r"(n) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(gsrc), "n"(BYTES), "r"(n) : "memory");
 }
 
 // Bound by instruction issue, not by HBM: the conversion costs about 5 packed
@@ -1090,7 +1079,7 @@ constexpr bool moduli_table_matches() {
 static_assert(moduli_table_matches(), "the gathers' compile-time moduli must be the plan's table");
 constexpr int kMinModuli = 8;
 constexpr int kMaxPassBlocks = 1023;  // K blocks of one exact INT32 pass (128^3 each, below 2^31)
-constexpr int kResidueBitsTarget = 46;  // operand bits kept by the default choice (INT8 slices keep 47)
+constexpr int kResidueBitsTarget = 46;  // the default choice: |X| <= 2^46, operands within 2^-48 as by six INT8 slices
 
 using u128 = unsigned __int128;
 
