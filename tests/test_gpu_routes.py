@@ -264,9 +264,16 @@ def test_more_groups_than_the_one_kernel_form_holds(xt, dev):
     assert np.linalg.norm(dev.get(dd, np.float64) - want) <= 4e-15 * np.linalg.norm(want)
 
 
-def test_short_of_scratch_the_one_kernel_form_runs(xt, dev):
+def test_short_of_scratch_the_one_kernel_form_runs():
     """With no memory for the residue planes (0.1 GB here) a long FP64 product runs in one
-    kernel, and the call that succeeded leaves no error text."""
+    kernel, and the call that succeeded leaves no error text.  In a process of its own,
+    whose scratch pool gives everything back."""
+    code = "import exatensor_b200 as X; X.device_init(0); import tests.test_gpu_routes as t; t.short_of_scratch(X)"
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
+def short_of_scratch(xt):
     from cuda.bindings import driver as cu
     m, n, k = 1400, 1100, 1290
     g = torch.Generator(device="cuda").manual_seed(1)
