@@ -360,12 +360,12 @@ int contract_impl(const int* cptrn, int dtk, int drank, const int* ddims, void* 
     //    to 30 us instead of 27 to 100 us for small ones).
     //  * R8 and C8 products picked plain but long enough run as residues with 15
     //    moduli, 51 or 52 operand bits, where that is predicted faster: 96/24
-    //    ladder 4.04 -> 1.57 ms, 1600^3 475 -> 186 us.  Residues keep those bits relative to
+    //    ladder 4.04 -> 1.55 ms, 1600^3 475 -> 185 us.  Residues keep those bits relative to
     //    a row's largest value, not of every element, so the GPU first counts how far
     //    the rows' values spread (GuardParams): where residues could be off by more
     //    than the bound of the FP64 sum, as with magnitudes that fall along the
     //    contracted index or many zeros, it runs the one-kernel form instead, for the
-    //    price of the counting pass (96/24 ladder 0.16 ms).  Measured relative to long double:
+    //    price of the counting pass (96/24 ladder 0.14 ms).  Measured relative to long double:
     //    uniform data 5e-17 against the plain sums' 5e-16 at K = 256 and 1.3e-15 at
     //    1600; normal data 4e-16 against 5e-16 and 1.4e-15.
     //  * A product picked for the tensor cores runs in one kernel where that is

@@ -250,7 +250,7 @@ struct GatherParams {
   void* planes;
   unsigned* rowE;      // per row: largest exponent field (slice modes read it; the
                        // split modes set it to 2047 for rows with a NaN or an infinity)
-  RowSpread* spread;   // row maxima that also count: [K split][row]; else null
+  RowSpread* spread;   // row maxima that also count: [row][K split]; else null
   int slices;
   int lanes_on_k;      // 1: consecutive k are contiguous in the source
   int vec;             // 1 (lanes_on_k): aligned 16-byte groups of k are contiguous and aligned in the source
@@ -734,7 +734,7 @@ __global__ void exps_kernel(const unsigned* __restrict__ rowE, int* __restrict__
 // C >= K / 4 is asked for as well.  Rows and columns with a NaN or an infinity (the
 // fix-up multiplies them in FP64) and rows of zeros do not count.
 struct GuardParams {
-  const RowSpread* a;        // [K split][row] of both operands
+  const RowSpread* a;        // [row][K split] of both operands
   const RowSpread* b;
   int64_t m, n;              // rows, columns
   int gy_a, gy_b;            // K splits
@@ -766,16 +766,20 @@ __global__ void __launch_bounds__(256) exps_pair_kernel(const unsigned* __restri
   if constexpr (GUARD) {
     // eight lanes merge a row's records
     unsigned miss[2][3] = {{0, 0, 0}, {0, 0, 0}};
+    __shared__ unsigned sm_miss[6];
+    if (threadIdx.x < 6) sm_miss[threadIdx.x] = 0;
+    __syncthreads();
     const int lane = threadIdx.x & 31, sub = lane & 7;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); 4 * w < G.m + G.n; w += warps) {
       const int64_t i = 4 * w + (lane >> 3);
       const bool in = i < G.m + G.n, col = i >= G.m;
-      const int64_t r = col ? i - G.m : i, rows = col ? G.n : G.m;
+      const int splits = col ? G.gy_b : G.gy_a;
+      const RowSpread* rec = col ? G.b + (i - G.m) * splits : G.a + i * splits;
       RowSpread S{0ull, 0u, 0u};
       if (in)
 #pragma unroll 4
-        for (int y = sub; y < (col ? G.gy_b : G.gy_a); y += 8) spread_merge(S, ((col ? G.b : G.a) + y * rows)[r]);
+        for (int y = sub; y < splits; y += 8) spread_merge(S, rec[y]);
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) {
         const RowSpread T{__shfl_xor_sync(0xffffffffu, S.bins, o), __shfl_xor_sync(0xffffffffu, S.e, o), 0u};
@@ -796,9 +800,13 @@ __global__ void __launch_bounds__(256) exps_pair_kernel(const unsigned* __restri
 #pragma unroll
       for (int s = 0; s < 3; ++s) {
         const unsigned v = __reduce_max_sync(0xffffffffu, miss[o][s]);
-        if (lane == 0 && v) atomicMax(&G.words[3 * o + s], v);
+        if (lane == 0 && v) atomicMax(&sm_miss[3 * o + s], v);
       }
-    __threadfence();
+    __syncthreads();
+    if (threadIdx.x < 6 && sm_miss[threadIdx.x]) {
+      atomicMax(&G.words[threadIdx.x], sm_miss[threadIdx.x]);
+      __threadfence();
+    }
     __syncthreads();
     if (threadIdx.x == 0 && atomicAdd(&G.words[6], 1u) == gridDim.x - 1) {
       __threadfence();
@@ -1211,14 +1219,14 @@ __device__ __forceinline__ void rowmax_body(const GatherParams& P, int64_t rowti
       if constexpr (SPREAD) {
 #pragma unroll
         for (int i = 1; i < KS; ++i) spread_merge(S, sm_spread[tid + i * TM]);
-        P.spread[(int64_t)ky * P.rows + m0 + tid] = S;
+        P.spread[(m0 + tid) * kstep + ky] = S;
       }
     }
     return;
   }
   if constexpr (SPREAD) {
     // half a warp per row: a thread counts in TM / 16 rows only (16 rows a thread, as
-    // below, take 128 registers: 200 against 148 us for the 96/24 ladder)
+    // below, take 128 registers: 200 against 131 us for the 96/24 ladder)
     constexpr int KL = 16, RR = TM * KL / kGThreads, KR = TK / KL;
     const int kl = tid % KL, r0 = tid / KL;
     int64_t lmv[RR];
@@ -1255,7 +1263,7 @@ __device__ __forceinline__ void rowmax_body(const GatherParams& P, int64_t rowti
       const int64_t m = m0 + r0 + i * (kGThreads / KL);
       if (kl == 0 && m < P.rows) {
         if (T.e) atomicMax(&P.rowE[m], T.e);
-        P.spread[(int64_t)ky * P.rows + m] = T;
+        P.spread[m * kstep + ky] = T;
       }
     }
     return;
