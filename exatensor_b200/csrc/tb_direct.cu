@@ -110,10 +110,8 @@ const std::vector<TileShape>& shapes(int dtk) {
 
 }  // namespace
 
-int direct_plan(const Matricization& Z, int dtk, const void* d, const void* l, const void* r, DirectPlan* out,
-                int force_variant, int force_split, int force_box) {
-  return plan_direct(Z, elem_bytes(dtk), is_complex(dtk), d, l, r, shapes(dtk), num_sms(), out, force_variant,
-                     force_split, force_box);
+int direct_plan(const Matricization& Z, int dtk, const void* d, const void* l, const void* r, DirectPlan* out) {
+  return plan_direct(Z, elem_bytes(dtk), is_complex(dtk), d, l, r, shapes(dtk), num_sms(), out);
 }
 
 int run_direct(const DirectPlan& plan, int dtk, double ar, double ai, bool accumulate, int lconj, int rconj,

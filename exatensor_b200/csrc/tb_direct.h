@@ -7,8 +7,7 @@
 namespace tb {
 
 // plan_direct over the kernels' tile shapes on the current device.
-int direct_plan(const Matricization& Z, int dtk, const void* d, const void* l, const void* r, DirectPlan* out,
-                int force_variant = -1, int force_split = 0, int force_box = -1);
+int direct_plan(const Matricization& Z, int dtk, const void* d, const void* l, const void* r, DirectPlan* out);
 // Launches it; alpha as the plain method takes it (real kinds: ai = 0).  `when` (R8, C8): a
 // device word; the kernel does nothing unless it is set.
 int run_direct(const DirectPlan& plan, int dtk, double ar, double ai, bool accumulate, int lconj, int rconj,

@@ -110,7 +110,8 @@ struct DirectPlan {
 // Returns TB_ERR_NOT_IMPLEMENTED for what it leaves to the other methods: more
 // than 2^30 rows, columns or contracted values, more index groups than its
 // parameter block holds, or an output that overlaps an operand.  The forced
-// values (>= 0; split > 0) pin the tile shape, K split and row boxes.
+// values (>= 0; split > 0) pin the tile shape, K split and row boxes (the CPU
+// replay of the index arithmetic goes through all of them).
 int plan_direct(const Matricization& Z, int es, bool cplx, const void* d, const void* l, const void* r,
                 const std::vector<TileShape>& shapes, int sms, DirectPlan* out, int force_variant = -1,
                 int force_split = 0, int force_box = -1);
